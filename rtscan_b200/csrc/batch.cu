@@ -40,6 +40,9 @@
 #include <type_traits>
 #include <vector>
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include "batch_plan.h"
 #include "rts_internal.h"
 
@@ -81,6 +84,17 @@ struct BatchPass {
   uint32_t word_bytes;          // 4, passed at run time (see the mask loop of batch4_kernel)
   const uint2 *pre;             // shared positions: the pass's table word offsets of row r at pre[r - pre_row0]
   uint64_t pre_row0;
+  // tables of batch_rows_kernel in shared memory (rows_layout): byte offset
+  // of column c's first copy, bytes between copies and their number, byte
+  // offset of its positions past the lines; lines, bytes per table word
+  // offset in the lines and behind them, bytes in all
+  uint32_t t_base[kMaxCols], t_rep[kMaxCols], t_nrep[kMaxCols], t_over[kMaxCols];
+  uint32_t t_lines, t_mul[2], t_bytes;
+  bool t_ovf;                   // some column has positions past the lines
+  uint32_t nslots;              // queries of the pass
+  int first_bitmap;             // >= 0: query i of the pass writes bitmap first_bitmap + i
+  int tma;                      // the result lines leave by TMA
+  uint32_t cnt_mul[2];          // 1 and 65536, passed at run time (see batch_rows_kernel)
 };
 
 // Log-linear bucket of v >= 0 with M mantissa bits: v itself below 2^M,
@@ -516,6 +530,7 @@ void launch_one(const BatchPass &bp, int sm_count, cudaStream_t s) {
 }
 
 #include "batch4.cuh"
+#include "batch_rows.cuh"
 #include "batch_few.cuh"
 #include "sparse_d2h.cuh"
 
@@ -563,17 +578,55 @@ void launch_shape4(const BatchPass &bp, int groups, int sm_count, cudaStream_t s
   else launch_one4<CMAX, 4, W, false>(bp, sm_count, s);
 }
 
-// A pass fed by shared positions (256 or 512 slots, four columns or fewer).
-void launch_pre4(const BatchPass &bp, int groups, int warps, int sm_count, cudaStream_t s) {
-  if (warps == 8) {
-    if (groups == 16) launch_one4<4, 16, 8, true>(bp, sm_count, s);
-    else if (groups == 8) launch_one4<4, 8, 8, true>(bp, sm_count, s);
-    else launch_one4<4, 4, 8, true>(bp, sm_count, s);
-  } else {
-    if (groups == 16) launch_one4<4, 16, 16, true>(bp, sm_count, s);
-    else if (groups == 8) launch_one4<4, 8, 16, true>(bp, sm_count, s);
-    else launch_one4<4, 4, 16, true>(bp, sm_count, s);
+// Shared memory of one of two CTAs resident on an SM (228 KiB, 1 KiB each
+// for the system).
+constexpr size_t kRowsHalfSM = 113 * 1024;
+
+// A pass with a thread per row, fed by shared positions.
+template <int C, int G, bool OVF>
+void launch_rows_shape(const BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
+  static std::atomic<uint64_t> raised{0};
+  raise_smem_limit(batch_rows_kernel<C, G, OVF>, raised, 227 * 1024);
+  const size_t sm = kRowsBuffer + bp.t_bytes;
+  if (sm > 227 * 1024) throw Error(RTS_ERR_ARG, "batch pass exceeds shared memory");
+  int per = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_rows_kernel<C, G, OVF>, 256, sm) != cudaSuccess ||
+      per < 1) {
+    cudaGetLastError();
+    per = 1;
   }
+  const int halves = RowsShape<G>::kHalves;
+  const uint64_t want = bp.nblocks - bp.block_begin;
+  const int grid = halves * (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count * per / halves));
+  batch_rows_kernel<C, G, OVF><<<grid, 256, sm, s>>>(bp, map);
+}
+
+template <int G, bool OVF>
+void launch_rows_cols(const BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
+  switch (bp.ncols) {
+    case 1: launch_rows_shape<1, G, OVF>(bp, map, sm_count, s); break;
+    case 2: launch_rows_shape<2, G, OVF>(bp, map, sm_count, s); break;
+    case 3: launch_rows_shape<3, G, OVF>(bp, map, sm_count, s); break;
+    default: launch_rows_shape<4, G, OVF>(bp, map, sm_count, s); break;
+  }
+}
+
+template <int G>
+void launch_rows_groups(const BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
+  if (bp.t_ovf) launch_rows_cols<G, true>(bp, map, sm_count, s);
+  else launch_rows_cols<G, false>(bp, map, sm_count, s);
+}
+
+void launch_rows(BatchPass &bp, int groups, int sm_count, cudaStream_t s) {
+  rows_layout(bp, groups, kRowsHalfSM);
+  bp.cnt_mul[0] = 1;
+  bp.cnt_mul[1] = 65536;
+  CUtensorMap map;
+  memset(&map, 0, sizeof map);
+  bp.tma = bp.first_bitmap >= 0 && rows_tensor_map(bp, bp.out + (uint64_t)bp.first_bitmap * bp.stride_words, &map);
+  if (groups == 16) launch_rows_groups<16>(bp, map, sm_count, s);
+  else if (groups == 8) launch_rows_groups<8>(bp, map, sm_count, s);
+  else launch_rows_groups<4>(bp, map, sm_count, s);
 }
 
 // Rows per block of a variant-4 pass shape.
@@ -1138,11 +1191,13 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
       blob.resize(blob.size() + (size_t)(bp.m[c] + 1) * Gp, 0u);
     }
     std::vector<uint32_t> free_mask((size_t)C * Gp, 0u);  // slots leaving column c unconstrained
-    for (int slot = 0; slot < (int)pp.qs.size(); slot++) {
+    auto slot_of = [&](int i) { return variant == 4 ? rows_slot(i) : i; };
+    for (int i = 0; i < (int)pp.qs.size(); i++) {
+      const int slot = slot_of(i);
       const uint32_t bit = 1u << (slot & 31);
       const int grp = slot >> 5;
       for (int c = 0; c < C; c++) free_mask[(size_t)c * Gp + grp] |= bit;
-      const NormQuery &q = norm[pp.qs[slot]];
+      const NormQuery &q = norm[pp.qs[i]];
       for (size_t k = 0; k < q.cols.size(); k++) {
         const int c = (int)(std::find(pp.cols.begin(), pp.cols.end(), q.cols[k]) - pp.cols.begin());
         const std::vector<uint32_t> &Bc = B[c];
@@ -1199,12 +1254,17 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
       memcpy(blob.data() + bp.bkt_off[c], bk.data(), bk.size() * 2);
     }
     bp.slot_off = (uint32_t)blob.size();
-    for (int slot = 0; slot < 32 * Gp; slot++) {
-      uint32_t o = 0xFFFFFFFFu;
-      if (slot < (int)pp.qs.size()) o = out_index ? (uint32_t)out_index[pp.qs[slot]] : (uint32_t)pp.qs[slot];
-      blob.push_back(o);
+    blob.resize(blob.size() + 32 * (size_t)Gp, 0xFFFFFFFFu);
+    bool in_order = true;
+    for (int i = 0; i < (int)pp.qs.size(); i++) {
+      const int o = out_index ? out_index[pp.qs[i]] : pp.qs[i];
+      blob[bp.slot_off + slot_of(i)] = (uint32_t)o;
+      if (i == 0) bp.first_bitmap = o;
+      else in_order = in_order && o == bp.first_bitmap + i;
     }
+    if (!in_order) bp.first_bitmap = -1;
     bp.blob_words = (uint32_t)blob.size();
+    bp.nslots = (uint32_t)pp.qs.size();
     for (int c = 0; c < C; c++) bp.col[c] = ctx->cols[pp.cols[c]];
     b.cmax = C <= 4 ? 4 : 8;
     b.variant = variant;
@@ -1366,7 +1426,9 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
     if (pre && b.pre_slot >= 0) {
       bp.pre = static_cast<const uint2 *>(scratch) + (uint64_t)b.pre_slot * pre_stride(pre_rows);
       bp.pre_row0 = row_begin;
-      launch_pre4(bp, b.groups, b.warps, ctx->sm_count, s);
+      bp.block_begin = row_begin / rows_block_rows(b.groups);
+      bp.nblocks = (row_end + rows_block_rows(b.groups) - 1) / rows_block_rows(b.groups);
+      launch_rows(bp, b.groups, ctx->sm_count, s);
     } else if (b.variant == 4) {
       if (b.cmax == 4) {
         if (b.warps == 8) launch_shape4<4, 8>(bp, b.groups, ctx->sm_count, s);
@@ -1525,6 +1587,8 @@ void batch_plan_drop(BatchPlan &plan, int qi, std::vector<uint32_t> &blob_words)
   const int64_t w = plan.where[qi];
   plan.where[qi] = INT64_MIN;
   if (w >= 0) {
+    for (auto &b : plan.passes)  // the pass's bitmaps are no longer all written
+      if (!b.few && (size_t)w >= b.off && (size_t)w < b.off + b.bp.blob_words) b.bp.first_bitmap = -1;
     plan.blob[w] = 0xFFFFFFFFu;
     blob_words.push_back((uint32_t)w);
     return;
