@@ -58,6 +58,16 @@ constexpr int kStageWords = kSlots * kTilesPerBlock;  // per warp
 template <int CMAX>
 constexpr int kPosWords = 36 * CMAX;  // per warp: 32 rows + one padding row per 8
 
+// Tables of a part of a pass of batch_rows_kernel in shared memory
+// (rows_layout): byte offset of column c's first copy, bytes between copies
+// and their number, byte offset of its positions past the lines; lines,
+// bytes per table word offset in the lines and behind them, bytes in all.
+struct RowsLayout {
+  uint32_t t_base[kMaxCols], t_rep[kMaxCols], t_nrep[kMaxCols], t_over[kMaxCols];
+  uint32_t t_lines, t_mul[2], t_bytes;
+  bool t_ovf;  // some column has positions past the lines
+};
+
 struct BatchPass {
   const uint32_t *col[kMaxCols];
   uint32_t m[kMaxCols];         // boundaries of column c
@@ -82,19 +92,18 @@ struct BatchPass {
   uint64_t nblocks;             // end of the range, in blocks
   int vec_store;                // bitmaps 16-byte aligned (out and stride)
   uint32_t word_bytes;          // 4, passed at run time (see the mask loop of batch4_kernel)
-  const uint2 *pre;             // shared positions: the pass's table word offsets of row r at pre[r - pre_row0]
-  uint64_t pre_row0;
-  // tables of batch_rows_kernel in shared memory (rows_layout): byte offset
-  // of column c's first copy, bytes between copies and their number, byte
-  // offset of its positions past the lines; lines, bytes per table word
-  // offset in the lines and behind them, bytes in all
-  uint32_t t_base[kMaxCols], t_rep[kMaxCols], t_nrep[kMaxCols], t_over[kMaxCols];
-  uint32_t t_lines, t_mul[2], t_bytes;
-  bool t_ovf;                   // some column has positions past the lines
+  // batch_rows_kernel: shared positions (the pass's table word offsets of row
+  // r at pre[r - row_begin], or two uint2 per row over more than four
+  // columns), the tables of the pass's parts, table words per position
+  const uint2 *pre;
+  uint64_t row_begin;
+  RowsLayout lay[2];
+  uint32_t groups;
+  uint32_t split;               // CTAs of the first part
   uint32_t nslots;              // queries of the pass
   int first_bitmap;             // >= 0: query i of the pass writes bitmap first_bitmap + i
   int tma;                      // the result lines leave by TMA
-  uint32_t cnt_mul[2];          // 1 and 65536, passed at run time (see batch_rows_kernel)
+  uint32_t cnt_mul[2];          // 1 and 65536, passed at run time (see batch_rows_part)
 };
 
 // Log-linear bucket of v >= 0 with M mantissa bits: v itself below 2^M,
@@ -156,7 +165,7 @@ __device__ __forceinline__ uint32_t position(const BatchPass &p, const uint32_t 
 // a union position fixes the position in every pass), and reads all the
 // passes' table word offsets for it from one entry of a per-column map.
 // The passes then read four 16-bit offsets per row instead of searching
-// (batch4_kernel with PRE).  Pass column c is union column c.
+// (batch_rows_kernel).  Pass column c is union column c.
 constexpr int kMaxPrePasses = kMaxSharedPasses;
 constexpr uint32_t kPreMaxBuckets = 4096;  // per union column
 
@@ -179,14 +188,15 @@ struct PreCol {
 };
 
 struct PreParams {
-  PreCol c[4];
+  PreCol c[kMaxCols];
   int ncols;                   // the passes' columns
   int npass;                   // 1..kMaxPrePasses
   const uint32_t *blob;        // union blob (global): per column buckets | boundaries | map
   uint32_t blob_words;
   uint64_t row_begin, row_end;
-  uint2 *out;                  // out[q * stride + (row - row_begin)]: pass q's four offsets, two per word
-  uint64_t stride;             // pre_stride(row_end - row_begin)
+  uint2 *out;                  // out[q * stride + (row - row_begin) * W]: pass q's 4 * W offsets, two per word,
+                               // W = 1 for up to four columns, else 2
+  uint64_t stride;             // pre_stride(row_end - row_begin) * W
   int vec;                     // every column 8-byte aligned at row_begin
 };
 
@@ -232,7 +242,7 @@ __host__ __device__ __forceinline__ uint64_t pre_stride(uint64_t rows) { return 
 // 8-byte aligned columns (P.vec) load each column's pair as one uint2 and
 // store each pass's pair as one uint4, without per-row checks.
 template <int U, int NW>
-__global__ void __launch_bounds__(kPreThreads, NW == 1 ? 2 : 1) pre_kernel(const __grid_constant__ PreParams P) {
+__global__ void __launch_bounds__(kPreThreads, NW == 1 && U <= 4 ? 2 : 1) pre_kernel(const __grid_constant__ PreParams P) {
   extern __shared__ __align__(16) uint32_t smem[];
   for (uint32_t i = threadIdx.x; i < P.blob_words; i += blockDim.x) smem[i] = __ldg(P.blob + i);
   __syncthreads();
@@ -257,13 +267,14 @@ __global__ void __launch_bounds__(kPreThreads, NW == 1 ? 2 : 1) pre_kernel(const
     }
     // map entries of every row and column; the searches of the thread's rows
     // and columns are independent, so their shared-memory loads overlap
-    uint32_t e[kPrePairs][2][4][NW];
+    constexpr int W = U <= 4 ? 1 : 2;
+    uint32_t e[kPrePairs][2][4 * W][NW];
 #pragma unroll
     for (int j = 0; j < kPrePairs; j++)
 #pragma unroll
       for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < 4 * W; c++) {
           if (c < U) {
             const uint32_t *ent = smem + P.c[c].map_off + pre_position(P.c[c], smem, x[j][h][c]) * NW;
             if (NW == 2) {
@@ -286,17 +297,28 @@ __global__ void __launch_bounds__(kPreThreads, NW == 1 ? 2 : 1) pre_kernel(const
         if (q >= P.npass) break;
         const int w = q >> 1;
         const uint32_t sel = (q & 1) ? 0x7632u : 0x5410u;  // the pass's halves of two entries
-        uint2 o[2];
+        uint2 o[2][W];
 #pragma unroll
         for (int h = 0; h < 2; h++)
-          o[h] = make_uint2(__byte_perm(e[j][h][0][w], e[j][h][1][w], sel),
-                            __byte_perm(e[j][h][2][w], e[j][h][3][w], sel));
-        uint2 *dst = P.out + q * P.stride + (row - P.row_begin);
+#pragma unroll
+          for (int i = 0; i < W; i++)
+            o[h][i] = make_uint2(__byte_perm(e[j][h][4 * i][w], e[j][h][4 * i + 1][w], sel),
+                                 __byte_perm(e[j][h][4 * i + 2][w], e[j][h][4 * i + 3][w], sel));
+        uint2 *dst = P.out + q * P.stride + (row - P.row_begin) * W;
         if (full) {
-          *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
+          if (W == 1) {
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0][0].x, o[0][0].y, o[1][0].x, o[1][0].y);
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+              reinterpret_cast<uint4 *>(dst)[h] = make_uint4(o[h][0].x, o[h][0].y, o[h][W - 1].x, o[h][W - 1].y);
+          }
         } else {
-          if (row < P.row_end) dst[0] = o[0];
-          if (row + 1 < P.row_end) dst[1] = o[1];
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            if (row + h < P.row_end)
+#pragma unroll
+              for (int i = 0; i < W; i++) dst[h * W + i] = o[h][i];
         }
       }
     }
@@ -553,14 +575,14 @@ size_t pass_smem4(size_t blob_words, int cmax, int groups, int warps) {
   return groups == 4 ? smem_bytes4<8, 4, 16>(w) : groups == 8 ? smem_bytes4<8, 8, 16>(w) : smem_bytes4<8, 16, 16>(w);
 }
 
-template <int CMAX, int GV, int W, bool PRE>
+template <int CMAX, int GV, int W>
 void launch_one4(const BatchPass &bp, int sm_count, cudaStream_t s) {
   static std::atomic<uint64_t> raised{0};
-  raise_smem_limit(batch4_kernel<CMAX, GV, W, PRE>, raised, 227 * 1024);
+  raise_smem_limit(batch4_kernel<CMAX, GV, W>, raised, 227 * 1024);
   const size_t sm = smem_bytes4<CMAX, GV, W>(bp.blob_words);
   if (sm > 227 * 1024) throw Error(RTS_ERR_ARG, "batch pass exceeds shared memory");
   int per = 1;  // CTAs per SM: one, or two 8-warp CTAs when the shared memory holds both
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch4_kernel<CMAX, GV, W, PRE>, W * 32, sm) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch4_kernel<CMAX, GV, W>, W * 32, sm) !=
           cudaSuccess ||
       per < 1) {
     cudaGetLastError();
@@ -568,14 +590,14 @@ void launch_one4(const BatchPass &bp, int sm_count, cudaStream_t s) {
   }
   const uint64_t want = bp.nblocks - bp.block_begin;
   const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count * per));
-  batch4_kernel<CMAX, GV, W, PRE><<<grid, W * 32, sm, s>>>(bp);
+  batch4_kernel<CMAX, GV, W><<<grid, W * 32, sm, s>>>(bp);
 }
 
 template <int CMAX, int W>
 void launch_shape4(const BatchPass &bp, int groups, int sm_count, cudaStream_t s) {
-  if (groups == 16) launch_one4<CMAX, 16, W, false>(bp, sm_count, s);
-  else if (groups == 8) launch_one4<CMAX, 8, W, false>(bp, sm_count, s);
-  else launch_one4<CMAX, 4, W, false>(bp, sm_count, s);
+  if (groups == 16) launch_one4<CMAX, 16, W>(bp, sm_count, s);
+  else if (groups == 8) launch_one4<CMAX, 8, W>(bp, sm_count, s);
+  else launch_one4<CMAX, 4, W>(bp, sm_count, s);
 }
 
 // Shared memory of one of two CTAs resident on an SM (228 KiB, 1 KiB each
@@ -584,10 +606,10 @@ constexpr size_t kRowsHalfSM = 113 * 1024;
 
 // A pass with a thread per row, fed by shared positions.
 template <int C, int G, bool OVF>
-void launch_rows_shape(const BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
+void launch_rows_shape(BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
   static std::atomic<uint64_t> raised{0};
   raise_smem_limit(batch_rows_kernel<C, G, OVF>, raised, 227 * 1024);
-  const size_t sm = kRowsBuffer + bp.t_bytes;
+  const size_t sm = kRowsBuffer + std::max(bp.lay[0].t_bytes, bp.lay[1].t_bytes);
   if (sm > 227 * 1024) throw Error(RTS_ERR_ARG, "batch pass exceeds shared memory");
   int per = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_rows_kernel<C, G, OVF>, 256, sm) != cudaSuccess ||
@@ -595,36 +617,56 @@ void launch_rows_shape(const BatchPass &bp, const CUtensorMap &map, int sm_count
     cudaGetLastError();
     per = 1;
   }
-  const int halves = RowsShape<G>::kHalves;
-  const uint64_t want = bp.nblocks - bp.block_begin;
-  const int grid = halves * (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count * per / halves));
-  batch_rows_kernel<C, G, OVF><<<grid, 256, sm, s>>>(bp, map);
+  // CTAs of the parts: a part of eight groups has twice the work of one of four
+  const uint64_t rows = bp.nrows - bp.row_begin, all = (uint64_t)sm_count * per;
+  const uint64_t blocks8 = std::max<uint64_t>(1, (rows + 1023) / 1024);
+  const uint64_t blocks4 = std::max<uint64_t>(1, (rows + 2047) / 2048);
+  const uint32_t n0 = (uint32_t)(G == 4    ? std::min(blocks4, all)
+                                 : G == 8  ? std::min(blocks8, all)
+                                 : G == 12 ? std::min(blocks8, std::max<uint64_t>(1, all * 2 / 3))
+                                           : std::min(blocks8, std::max<uint64_t>(1, all / 2)));
+  const uint32_t n1 = (uint32_t)(G <= 8    ? 0
+                                 : G == 12 ? std::min(blocks4, std::max<uint64_t>(1, all - n0))
+                                           : n0);
+  bp.split = n0;
+  batch_rows_kernel<C, G, OVF><<<n0 + n1, 256, sm, s>>>(bp, map);
 }
 
 template <int G, bool OVF>
-void launch_rows_cols(const BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
+void launch_rows_cols(BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
   switch (bp.ncols) {
     case 1: launch_rows_shape<1, G, OVF>(bp, map, sm_count, s); break;
     case 2: launch_rows_shape<2, G, OVF>(bp, map, sm_count, s); break;
     case 3: launch_rows_shape<3, G, OVF>(bp, map, sm_count, s); break;
-    default: launch_rows_shape<4, G, OVF>(bp, map, sm_count, s); break;
+    case 4: launch_rows_shape<4, G, OVF>(bp, map, sm_count, s); break;
+    case 5: launch_rows_shape<5, G, OVF>(bp, map, sm_count, s); break;
+    case 6: launch_rows_shape<6, G, OVF>(bp, map, sm_count, s); break;
+    case 7: launch_rows_shape<7, G, OVF>(bp, map, sm_count, s); break;
+    default: launch_rows_shape<8, G, OVF>(bp, map, sm_count, s); break;
   }
 }
 
 template <int G>
-void launch_rows_groups(const BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
-  if (bp.t_ovf) launch_rows_cols<G, true>(bp, map, sm_count, s);
+void launch_rows_groups(BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
+  if (bp.lay[0].t_ovf || bp.lay[1].t_ovf) launch_rows_cols<G, true>(bp, map, sm_count, s);
   else launch_rows_cols<G, false>(bp, map, sm_count, s);
 }
 
-void launch_rows(BatchPass &bp, int groups, int sm_count, cudaStream_t s) {
-  rows_layout(bp, groups, kRowsHalfSM);
+void launch_rows(BatchPass &bp, int sm_count, cudaStream_t s) {
+  const int groups = (int)bp.groups;
+  // parts in use: a 512-slot pass of up to 384 queries needs only four
+  // groups past its first eight
+  const bool twelve = groups == 16 && bp.nslots <= 384;
+  memset(bp.lay, 0, sizeof bp.lay);
+  bp.lay[0] = rows_layout(bp, groups, std::min(groups, 8), kRowsHalfSM);
+  if (twelve) bp.lay[1] = rows_layout(bp, groups, 4, kRowsHalfSM);
   bp.cnt_mul[0] = 1;
   bp.cnt_mul[1] = 65536;
   CUtensorMap map;
   memset(&map, 0, sizeof map);
   bp.tma = bp.first_bitmap >= 0 && rows_tensor_map(bp, bp.out + (uint64_t)bp.first_bitmap * bp.stride_words, &map);
-  if (groups == 16) launch_rows_groups<16>(bp, map, sm_count, s);
+  if (twelve) launch_rows_groups<12>(bp, map, sm_count, s);
+  else if (groups == 16) launch_rows_groups<16>(bp, map, sm_count, s);
   else if (groups == 8) launch_rows_groups<8>(bp, map, sm_count, s);
   else launch_rows_groups<4>(bp, map, sm_count, s);
 }
@@ -805,13 +847,21 @@ struct BatchPlan {
     int groups;   // 32-slot groups of the pass (table words per position)
     bool few;     // at most kFewMaxQueries queries: tested term by term (batch_few_kernel), no tables
     FewPass fp;
-    int pre_slot = -1;  // shared positions: this pass's slot in the scratch, or -1 (it searches)
+    int pre_slot = -1;  // shared positions: this pass's slot in the scratch, or -1
+    // a further group of passes sharing positions, and the slot in it (both
+    // -1: the pass searches)
+    int group = -1, group_slot = -1;
+  };
+  struct Group {
+    PreParams pre;
+    size_t off;  // word offset of its union data in `blob`
   };
   std::vector<Pass> passes;
   std::vector<uint32_t> blob;
   // shared positions of the passes with a pre_slot (npass 0: none)
   PreParams pre;
   size_t pre_off = 0;  // word offset of the union boundaries, buckets and maps in `blob`
+  std::vector<Group> groups;
   // batch_plan_drop: per query index, where its slot is (built at the first
   // drop): the blob word of a table-pass slot, or -(1 + pass) for a
   // term-by-term pass, or INT64_MIN when the plan does not hold it
@@ -932,7 +982,8 @@ uint64_t pre_bucket_start(uint32_t M, uint32_t L, uint32_t k) {
 // ones with the smallest L that fits; the one whose boundaries need the
 // fewest search steps in all wins (the query bounds sit where the rows
 // are dense), fewer buckets on a tie.
-std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc) {
+std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc,
+                                  uint32_t max_buckets = kPreMaxBuckets) {
   const uint32_t m = (uint32_t)B.size();
   pc.m = m;
   pc.origin = m && B[0] > 0 ? B[0] - 1 : 0;
@@ -974,7 +1025,7 @@ std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc) {
   uint32_t bestM, bestL, bestN;
   {
     uint32_t L = 0;
-    while ((vmax >> L) >= kPreMaxBuckets) L++;
+    while ((vmax >> L) >= max_buckets) L++;
     bestM = 31;
     bestL = L;
     bestN = (vmax >> L) + 1;
@@ -987,7 +1038,7 @@ std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc) {
       t.L = L;
       t.nbk = 0xFFFFFFFFu;
       const uint32_t nbk = pre_bucket(t, B.back()) + 1;
-      if (nbk > kPreMaxBuckets) continue;
+      if (nbk > max_buckets) continue;
       const double cost = cost_of(M, L, nbk);
       if (cost < best_cost || (cost == best_cost && nbk < bestN)) {
         best_cost = cost;
@@ -1038,22 +1089,9 @@ void move_column(BatchPass &dst, int c, const BatchPass &src, int s) {
 // pass's boundaries are a subset of the union, so the pass position of
 // union position k is the number of its boundaries <= B_u[k-1]).  Appended
 // to the plan blob; other plans are left as they are.
-void plan_shared_positions(BatchPlan &plan) {
-  plan.pre.npass = 0;
-  std::vector<int> which;
-  for (size_t i = 0; i < plan.passes.size() && (int)which.size() < kMaxPrePasses; i++) {
-    const BatchPlan::Pass &b = plan.passes[i];
-    if (b.few || b.variant != 4 || b.cmax != 4) continue;
-    if (!which.empty()) {
-      const BatchPass &f = plan.passes[which[0]].bp;
-      if (b.bp.ncols != f.ncols) continue;
-      bool same = true;
-      for (int c = 0; c < f.ncols; c++) same = same && std::find(b.bp.col, b.bp.col + b.bp.ncols, f.col[c]) != b.bp.col + b.bp.ncols;
-      if (!same) continue;
-    }
-    which.push_back((int)i);
-  }
-  if (which.empty()) return;
+// Passes `which` (the same columns each) share: fills P and appends the union
+// data to the plan blob; false (the plan unchanged) when it does not fit.
+bool share_group(BatchPlan &plan, const std::vector<int> &which, PreParams &P, size_t *off) {
   const int U = plan.passes[which[0]].bp.ncols;
   const int npass = (int)which.size(), NW = (npass + 1) / 2;
   std::vector<std::vector<uint32_t>> Bu(U);
@@ -1075,17 +1113,17 @@ void plan_shared_positions(BatchPlan &plan) {
       Bu[c].swap(merged);
     }
   }
-  PreParams P;
   memset(&P, 0, sizeof P);
   P.ncols = U;
   P.npass = npass;
   std::vector<uint32_t> ub;  // offsets relative to its own start
   for (int c = 0; c < U; c++) {
     const std::vector<uint32_t> &B = Bu[c];  // sorted and distinct
-    if (B.size() > 0xFFFFu) return;  // bucket entries hold 16-bit positions
+    if (B.size() > 0xFFFFu) return false;  // bucket entries hold 16-bit positions
     PreCol &pc = P.c[c];
     pc.col = ordered[0].col[c];
-    const std::vector<uint32_t> ent = pre_buckets(B, pc);
+    // (eight columns of 4096 buckets would leave no room for their maps)
+    const std::vector<uint32_t> ent = pre_buckets(B, pc, U <= 4 ? kPreMaxBuckets : kPreMaxBuckets / 2);
     pc.bkt_off = (uint32_t)ub.size();
     ub.insert(ub.end(), ent.begin(), ent.end());
     pc.bnd_off = (uint32_t)ub.size();
@@ -1101,22 +1139,61 @@ void plan_shared_positions(BatchPlan &plan) {
       for (size_t k = 0; k <= B.size(); k++) {
         if (k > 0)
           while (j < mp && Bp[j] <= B[k - 1]) j++;
-        const uint64_t off = (uint64_t)ordered[q].tab_off[c] + (uint64_t)j * b.groups;
-        if (off > 0xFFFFu) return;  // table offsets are 16-bit in the map
-        ub[pc.map_off + k * NW + q / 2] |= (uint32_t)off << (16 * (q & 1));
+        const uint64_t o = (uint64_t)ordered[q].tab_off[c] + (uint64_t)j * b.groups;
+        if (o > 0xFFFFu) return false;  // table offsets are 16-bit in the map
+        ub[pc.map_off + k * NW + q / 2] |= (uint32_t)o << (16 * (q & 1));
       }
     }
   }
-  if (ub.size() * 4 > 200 * 1024) return;  // the pre kernel's shared memory
+  if (ub.size() * 4 > 200 * 1024) return false;  // the pre kernel's shared memory
   P.blob_words = (uint32_t)ub.size();
-  plan.pre = P;
-  for (int q = 0; q < npass; q++) {
-    plan.passes[which[q]].bp = ordered[q];
-    plan.passes[which[q]].pre_slot = q;
-  }
+  for (int q = 0; q < npass; q++) plan.passes[which[q]].bp = ordered[q];
   while (plan.blob.size() % 4) plan.blob.push_back(0);
-  plan.pre_off = plan.blob.size();
+  *off = plan.blob.size();
   plan.blob.insert(plan.blob.end(), ub.begin(), ub.end());
+  return true;
+}
+
+// The first passes over the same four columns or fewer (up to kMaxPrePasses)
+// become the plan's first group; the other table passes make further groups
+// of passes over the same columns (up to two when they have more than four),
+// which run one after another and use the same scratch.
+void plan_shared_positions(BatchPlan &plan) {
+  plan.pre.npass = 0;
+  auto fits = [&](size_t i, int cmax) {
+    const BatchPlan::Pass &b = plan.passes[i];
+    return !b.few && b.variant == 4 && b.pre_slot < 0 && b.group < 0 && b.cmax <= cmax;
+  };
+  auto alike = [&](size_t i, size_t first) {
+    const BatchPass &b = plan.passes[i].bp, &f = plan.passes[first].bp;
+    if (b.ncols != f.ncols) return false;
+    for (int c = 0; c < f.ncols; c++)
+      if (std::find(b.col, b.col + b.ncols, f.col[c]) == b.col + b.ncols) return false;
+    return true;
+  };
+  auto gather = [&](size_t first, int cmax, int most) {
+    std::vector<int> which;
+    for (size_t i = first; i < plan.passes.size() && (int)which.size() < most; i++)
+      if (fits(i, cmax) && (which.empty() || alike(i, which[0]))) which.push_back((int)i);
+    return which;
+  };
+  const std::vector<int> which = gather(0, 4, kMaxPrePasses);
+  if (!which.empty() && share_group(plan, which, plan.pre, &plan.pre_off))
+    for (size_t q = 0; q < which.size(); q++) plan.passes[which[q]].pre_slot = (int)q;
+  else
+    plan.pre.npass = 0;
+  for (size_t i = 0; i < plan.passes.size(); i++) {
+    if (!fits(i, 8)) continue;
+    const int cmax = plan.passes[i].cmax;
+    const std::vector<int> w = gather(i, cmax, cmax == 4 ? kMaxPrePasses : 2);
+    BatchPlan::Group g;
+    if (!share_group(plan, w, g.pre, &g.off)) continue;
+    for (size_t q = 0; q < w.size(); q++) {
+      plan.passes[w[q]].group = (int)plan.groups.size();
+      plan.passes[w[q]].group_slot = (int)q;
+    }
+    plan.groups.push_back(g);
+  }
 }
 
 // Passes for the kernel queries `which` (indices into norm); query qi writes
@@ -1265,6 +1342,7 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
     if (!in_order) bp.first_bitmap = -1;
     bp.blob_words = (uint32_t)blob.size();
     bp.nslots = (uint32_t)pp.qs.size();
+    bp.groups = (uint32_t)Gp;
     for (int c = 0; c < C; c++) bp.col[c] = ctx->cols[pp.cols[c]];
     b.cmax = C <= 4 ? 4 : 8;
     b.variant = variant;
@@ -1326,14 +1404,23 @@ void launch_pre_nw(rts_ctx *ctx, const PreParams &P, cudaStream_t s) {
   }
 }
 
+uint64_t pre_pass_stride(const PreParams &P, uint64_t rows) { return pre_stride(rows) * (P.ncols <= 4 ? 1 : 2); }
+
 void launch_pre(rts_ctx *ctx, PreParams P, cudaStream_t s) {
-  P.stride = pre_stride(P.row_end - P.row_begin);
+  P.stride = pre_pass_stride(P, P.row_end - P.row_begin);
   P.vec = ((uintptr_t)P.out & 15) == 0;
   for (int c = 0; c < P.ncols; c++) P.vec = P.vec && ((uintptr_t)(P.c[c].col + P.row_begin) & 7) == 0;
-  if (P.npass <= 2)
-    launch_pre_nw<1>(ctx, P, s);
-  else
-    launch_pre_nw<2>(ctx, P, s);
+  if (P.ncols <= 4) {
+    if (P.npass <= 2) launch_pre_nw<1>(ctx, P, s);
+    else launch_pre_nw<2>(ctx, P, s);
+    return;
+  }
+  switch (P.ncols) {
+    case 5: launch_pre_shape<5, 1>(ctx, P, s); break;
+    case 6: launch_pre_shape<6, 1>(ctx, P, s); break;
+    case 7: launch_pre_shape<7, 1>(ctx, P, s); break;
+    default: launch_pre_shape<8, 1>(ctx, P, s); break;
+  }
 }
 
 // Launch every pass of `plan` (blob already on the device) over rows
@@ -1343,21 +1430,47 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
                 unsigned long long *counts, uint64_t row_begin, uint64_t row_end, void *scratch,
                 size_t scratch_bytes, cudaStream_t s) {
   int launches = 0;
-  // shared positions, when the caller's scratch holds them; else every pass
-  // searches its own
-  const uint64_t pre_rows = row_end > row_begin ? row_end - row_begin : 0;
-  const bool pre = plan.pre.npass > 0 && pre_rows > 0 && scratch &&
-                   (uint64_t)plan.pre.npass * pre_stride(pre_rows) * sizeof(uint2) <= scratch_bytes;
-  if (pre) {
-    PreParams P = plan.pre;
-    P.blob = dev_blob + plan.pre_off;
+  // the passes of each group that shares positions, when the caller's scratch
+  // holds them: the positions, then the passes (the scratch is the next
+  // group's after that); the others search their own
+  const uint64_t rows = row_end > row_begin ? row_end - row_begin : 0;
+  std::vector<char> done(plan.passes.size(), 0);
+  auto run_group = [&](const PreParams &pre, size_t off, auto &&slot_of) {
+    const uint64_t stride = pre_pass_stride(pre, rows);
+    if (pre.npass == 0 || rows == 0 || !scratch || (uint64_t)pre.npass * stride * sizeof(uint2) > scratch_bytes) return;
+    PreParams P = pre;
+    P.blob = dev_blob + off;
     P.row_begin = row_begin;
     P.row_end = row_end;
     P.out = static_cast<uint2 *>(scratch);
     launch_pre(ctx, P, s);
     launches++;
-  }
-  for (auto &b : plan.passes) {
+    for (size_t i = 0; i < plan.passes.size(); i++) {
+      const BatchPlan::Pass &b = plan.passes[i];
+      const int q = slot_of(b);
+      if (q < 0) continue;
+      BatchPass bp = b.bp;
+      bp.blob = dev_blob + b.off;
+      bp.out = out;
+      bp.stride_words = stride_words;
+      bp.counts = counts;
+      bp.nrows = row_end;
+      bp.words = words_for(ctx->nrows);
+      bp.vec_store = (((uintptr_t)out & 15) == 0 && stride_words % 4 == 0) ? 1 : 0;
+      bp.pre = P.out + (uint64_t)q * stride;
+      bp.row_begin = row_begin;
+      launch_rows(bp, ctx->sm_count, s);
+      launches++;
+      done[i] = 1;
+    }
+  };
+  run_group(plan.pre, plan.pre_off, [](const BatchPlan::Pass &b) { return b.pre_slot; });
+  for (size_t g = 0; g < plan.groups.size(); g++)
+    run_group(plan.groups[g].pre, plan.groups[g].off,
+              [g](const BatchPlan::Pass &b) { return b.group == (int)g ? b.group_slot : -1; });
+  for (size_t pi = 0; pi < plan.passes.size(); pi++) {
+    auto &b = plan.passes[pi];
+    if (done[pi]) continue;
     if (b.few && fused_each(b.fp)) {
       // one query (or two over few columns): the single-query scan kernel
       // over the range per query, which runs at HBM speed (the term-by-term
@@ -1423,13 +1536,7 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
     bp.vec_store = (((uintptr_t)out & 15) == 0 && stride_words % 4 == 0) ? 1 : 0;
     bp.word_bytes = 4;
     const bool w8 = ctx->batch_cfg.warps_per_cta == 8;
-    if (pre && b.pre_slot >= 0) {
-      bp.pre = static_cast<const uint2 *>(scratch) + (uint64_t)b.pre_slot * pre_stride(pre_rows);
-      bp.pre_row0 = row_begin;
-      bp.block_begin = row_begin / rows_block_rows(b.groups);
-      bp.nblocks = (row_end + rows_block_rows(b.groups) - 1) / rows_block_rows(b.groups);
-      launch_rows(bp, b.groups, ctx->sm_count, s);
-    } else if (b.variant == 4) {
+    if (b.variant == 4) {
       if (b.cmax == 4) {
         if (b.warps == 8) launch_shape4<4, 8>(bp, b.groups, ctx->sm_count, s);
         else launch_shape4<4, 16>(bp, b.groups, ctx->sm_count, s);
@@ -1492,7 +1599,10 @@ const uint32_t *upload_plan(rts_ctx *ctx, const BatchPlan &plan, cudaStream_t s,
 }
 
 size_t plan_pre_bytes(const BatchPlan &plan, uint64_t rows) {
-  return (size_t)plan.pre.npass * pre_stride(rows) * sizeof(uint2);
+  size_t need = (size_t)plan.pre.npass * pre_pass_stride(plan.pre, rows) * sizeof(uint2);
+  for (const auto &g : plan.groups)
+    need = std::max(need, (size_t)g.pre.npass * pre_pass_stride(g.pre, rows) * sizeof(uint2));
+  return need;
 }
 
 // The context's shared-position scratch for `bytes`, ordered after its last

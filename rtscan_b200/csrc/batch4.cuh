@@ -1,4 +1,5 @@
-// Batched kernel with table-driven passes of up to 512 queries (included by
+// Table passes that search their own positions, of up to 512 queries: the
+// passes of a plan whose shared positions do not fit the scratch (included by
 // batch.cu inside its anonymous namespace; uses BatchPass, position_fast(),
 // position() and kFull from there).
 //
@@ -28,8 +29,7 @@
 // measured 2.9 % faster per 1024-query step (passes reading shared
 // positions), 1.8 % faster for 400- and 512-query batches and 20-22 %
 // faster for 64- and 128-query ones.  For 512- and 256-slot passes over up
-// to 4 columns, and every pass reading shared positions, step 1 for the
-// next block runs inside step 2 (see the kernel).
+// to 4 columns step 1 for the next block runs inside step 2 (see the kernel).
 template <int GV, int W>
 struct V4Shape {
   static_assert(GV == 16 || GV == 8 || GV == 4, "512-, 256- or 128-slot passes");
@@ -135,11 +135,7 @@ __device__ __forceinline__ void transpose16x2(uint32_t (&x)[16]) {
   }
 }
 
-// PRE: the batch's positions were found once for all its passes
-// (pre_kernel in batch.cu), and this pass reads its rows' table word
-// offsets (four uint16 per row) from p.pre instead of searching; only for
-// the shapes that find positions a block ahead.
-template <int CMAX, int GV, int W, bool PRE>
+template <int CMAX, int GV, int W>
 __global__ void __launch_bounds__(W * 32, 16 / W) batch4_kernel(const __grid_constant__ BatchPass p) {
   using S = V4Shape<GV, W>;
   constexpr int kV4Threads = S::kThreads;
@@ -173,22 +169,15 @@ __global__ void __launch_bounds__(W * 32, 16 / W) batch4_kernel(const __grid_con
   // 16-bit pairs until the next step 1 writes them to shared memory, and the
   // column values are loaded one more block ahead.  Other shapes find the
   // positions of a block in its own step 1.
-  constexpr bool kAhead = (GV == 16 || GV == 8 || PRE) && CMAX <= 4;
-  static_assert(!PRE || (kAhead && CMAX == 4), "shared positions feed the 4-column look-ahead shapes");
-  uint32_t val[S::kRPT][CMAX];                    // column values of this thread's rows (PRE: packed offsets)
+  constexpr bool kAhead = (GV == 16 || GV == 8) && CMAX <= 4;
+  uint32_t val[S::kRPT][CMAX];                    // column values of this thread's rows
   uint32_t offn[kAhead ? S::kRPT : 1][(CMAX + 1) / 2];  // their table word offsets, two per register
   auto load_values = [&](uint64_t b) {
 #pragma unroll
     for (int h = 0; h < S::kRPT; h++) {
       const uint64_t row = b * S::kRows + threadIdx.x + h * kV4Threads;
-      if (PRE) {  // the row's four offsets, two per word, as find_offsets packs them
-        const uint2 w = row < p.nrows ? __ldg(p.pre + (row - p.pre_row0)) : make_uint2(0u, 0u);
-        val[h][0] = w.x;
-        val[h][1] = w.y;
-      } else {
 #pragma unroll
-        for (int c = 0; c < CMAX; c++) val[h][c] = (c < C && row < p.nrows) ? __ldg(p.col[c] + row) : 0u;
-      }
+      for (int c = 0; c < CMAX; c++) val[h][c] = (c < C && row < p.nrows) ? __ldg(p.col[c] + row) : 0u;
     }
   };
   // kAhead: latency hidden behind the masks, so the search with the fewest
@@ -265,16 +254,11 @@ __global__ void __launch_bounds__(W * 32, 16 / W) batch4_kernel(const __grid_con
   auto find_offsets = [&](uint64_t b) {  // kAhead: into offn
 #pragma unroll
     for (int h = 0; h < S::kRPT; h++) {
-      if (PRE) {
-        offn[h % (kAhead ? S::kRPT : 1)][0] = val[h][0];
-        offn[h % (kAhead ? S::kRPT : 1)][1 % ((CMAX + 1) / 2)] = val[h][1];
-      } else {
-        uint32_t off[CMAX];
-        row_offsets(b, h, off);
+      uint32_t off[CMAX];
+      row_offsets(b, h, off);
 #pragma unroll
-        for (int c = 0; c < CMAX; c += 2)
-          offn[h % (kAhead ? S::kRPT : 1)][c / 2] = off[c] | (c + 1 < CMAX ? off[c + 1] << 16 : 0u);
-      }
+      for (int c = 0; c < CMAX; c += 2)
+        offn[h % (kAhead ? S::kRPT : 1)][c / 2] = off[c] | (c + 1 < CMAX ? off[c + 1] << 16 : 0u);
     }
   };
   auto put_offsets = [&]() {  // kAhead: from offn

@@ -31,7 +31,7 @@
 //   * the buffer's 16-byte pieces are swizzled by row and tile so that phase
 //     A's 16-byte stores, phase B's 4-byte loads and stores and phase C's
 //     16-byte loads meet 32 banks.
-// A table position past the lines that fit (p.t_lines) has its row packed
+// A table position past the lines that fit (L.t_lines) has its row packed
 // behind them instead, once: correct, with bank conflicts.  Two CTAs per SM
 // hold about 648 lines each, so a column of a 512-slot pass that every
 // second query constrains twice overflows by a few positions.
@@ -45,25 +45,19 @@
 // 16-byte stores of eight lanes instead of TMA: 2.65 ms per 512-query pass;
 // 4-byte stores straight from phase B's registers (32-byte sectors of four
 // bitmaps per instruction): 4.7 ms.  All rows packed (no lines): 2.8 ms.
-template <int G>
+template <int KG>  // groups of a CTA
 struct RowsShape {
-  static_assert(G == 16 || G == 8 || G == 4, "512-, 256- or 128-slot passes");
-  static constexpr int kHalves = G == 16 ? 2 : 1;
-  static constexpr int kG = G / kHalves;                 // groups of a CTA
-  static constexpr int kQ = kG / 4;                      // 16-byte parts of a row's mask
+  static_assert(KG == 8 || KG == 4, "256 or 128 slots per CTA");
+  static constexpr int kQ = KG / 4;                      // 16-byte parts of a row's mask
   static constexpr int kLQ = kQ == 2 ? 1 : 0;
   static constexpr int kS = 8 / kQ;                      // table rows per 128-byte line
   static constexpr int kLS = 3 - kLQ;
-  static constexpr int kRPT = 32 / kG;                   // rows per thread and block
+  static constexpr int kRPT = 32 / KG;                   // rows per thread and block
   static constexpr int kRows = 256 * kRPT;               // rows per block
   static constexpr int kTiles = kRows / 32;
-  static constexpr int kLPQ = kTiles / 4;                // lanes per query in phase C
-  static constexpr int kQPI = 32 / kLPQ;                 // queries per store instruction
 };
 constexpr int kRowsBuffer = 32768;  // row masks, then result words
 
-// Rows per block of a pass of `groups` groups.
-constexpr uint64_t rows_block_rows(int groups) { return groups == 4 ? 2048 : 1024; }
 
 // Size and first column of the group that column c of C is in, with S slots
 // per line: groups are the powers of two of C, largest first, at most S.
@@ -125,33 +119,33 @@ __host__ __device__ inline int rows_slot(int i) {
   return (i & ~127) + 32 * ((i >> 1) & 3) + 2 * ((i & 127) >> 3) + (i & 1);
 }
 
-// OVF: some column has positions past the lines.
-template <int C, int G, bool OVF>
-__global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constant__ BatchPass p,
-                                                                      const __grid_constant__ CUtensorMap tmap) {
-  using R = RowsShape<G>;
+// One CTA's part of a pass: groups g0 .. g0 + KG - 1 on blocks bid, bid + nb,
+// ... of the range, with the tables laid out as L says.  OVF: some column
+// has positions past the lines.
+template <int C, int KG, bool OVF>
+__device__ __forceinline__ void batch_rows_part(const BatchPass &p, const RowsLayout &L, const CUtensorMap *tmap, int g0,
+                                                uint32_t bid, uint32_t nb) {
+  using R = RowsShape<KG>;
   constexpr int Q = R::kQ, S = R::kS;
   extern __shared__ __align__(1024) unsigned char rows_sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char *buf = rows_sm;
   const unsigned char *tables = rows_sm + kRowsBuffer;
-  const uint32_t nb = gridDim.x / R::kHalves;
-  const int half = R::kHalves == 2 && blockIdx.x >= nb;
-  const uint32_t bid = blockIdx.x - half * nb;
+  const uint64_t block_begin = p.row_begin / R::kRows, nblocks = (p.nrows + R::kRows - 1) / R::kRows;
 
-  // the half's tables (and their copies) and bitmaps
+  // the part's tables and their copies
   for (int c = 0; c < C; c++) {
-    const uint32_t *src = p.blob + p.tab_off[c] + half * R::kG;
+    const uint32_t *src = p.blob + p.tab_off[c] + g0;
     const uint32_t n = (p.m[c] + 1) * Q;
     for (uint32_t k = tid; k < n; k += 256) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src + (k / Q) * G) + k % Q);
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src + (k / Q) * p.groups) + k % Q);
       const uint32_t pos = k / Q;
       unsigned char *dst = rows_sm + kRowsBuffer + (k % Q) * 16;
-      if (!OVF || pos < p.t_lines) {
-        for (uint32_t r = 0; r < p.t_nrep[c]; r++)
-          *reinterpret_cast<uint4 *>(dst + p.t_base[c] + pos * 128 + r * p.t_rep[c]) = v;
+      if (!OVF || pos < L.t_lines) {
+        for (uint32_t r = 0; r < L.t_nrep[c]; r++)
+          *reinterpret_cast<uint4 *>(dst + L.t_base[c] + pos * 128 + r * L.t_rep[c]) = v;
       } else {
-        *reinterpret_cast<uint4 *>(dst + p.t_over[c] + (pos - p.t_lines) * (4 * R::kG)) = v;
+        *reinterpret_cast<uint4 *>(dst + L.t_over[c] + (pos - L.t_lines) * (4 * KG)) = v;
       }
     }
   }
@@ -162,16 +156,15 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
   const uint32_t hx = lane & (Q - 1), sb = (lane & 7) >> R::kLQ;
   uint32_t lc[OVF ? 1 : Q][C];  // byte offset of table word offset 0 of the k-th column, part s ^ hx
   uint32_t lim[C], lo[C];       // OVF: word offset of its first position past the lines, offset of those rows
-  constexpr uint32_t kMul = 128 / G, kMulOver = 4 * R::kG / G;  // bytes per table word offset
 #pragma unroll
   for (int k = 0; k < C; k++) {
     const int size = rows_group_size(C, S, k);
     const int c = rows_group_start(C, S, k) + ((k - rows_group_start(C, S, k)) ^ (sb & (size - 1)));
 #pragma unroll
     for (int s = 0; s < (OVF ? 1 : Q); s++)
-      lc[s][k] = p.t_base[c] + p.t_rep[c] * (sb >> rows_log2(size)) - p.tab_off[c] * kMul + ((s ^ hx) << 4);
-    lim[k] = p.tab_off[c] + p.t_lines * G;
-    lo[k] = p.t_over[c] - lim[k] * kMulOver + (hx << 4);
+      lc[s][k] = L.t_base[c] + L.t_rep[c] * (sb >> rows_log2(size)) - p.tab_off[c] * L.t_mul[0] + ((s ^ hx) << 4);
+    lim[k] = p.tab_off[c] + L.t_lines * p.groups;
+    lo[k] = L.t_over[c] - lim[k] * L.t_mul[1] + (hx << 4);
   }
   // a row's offsets come two to a word: the byte selector of the half of the
   // k-th column (the other half when sb is odd)
@@ -188,7 +181,7 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
   const int chunk = (2 * oct + (tl >> 2)) & 7;
   unsigned char *const mwr = buf + (Q == 2 ? h : oct >> 2) * 16384 + gl * 256 + (tl & 3) * 4;
   unsigned char *const mw0 = mwr + ((chunk ^ (2 * gl)) << 4), *const mw1 = mwr + 128 + ((chunk ^ (2 * gl) ^ 1) << 4);
-  const bool used = 256 * half + 128 * h < (int)p.nslots;
+  const bool used = 32 * g0 + 128 * h < (int)p.nslots;
   uint32_t cnt[16];  // matches of the lane's 32 slots, two 16-bit counters each
 #pragma unroll
   for (int j = 0; j < 16; j++) cnt[j] = 0;
@@ -205,37 +198,45 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
     for (int j = 0; j < 16; j++) cnt[j] = 0;
   };
 
+  // The rows' table word offsets, two per word.  Over up to four columns the
+  // next block's are loaded behind phase A; over more (16 bytes a row, too
+  // many registers to hold) they are only brought to L2 there.
   constexpr int kOffWords = C <= 4 ? 2 : 4;
-  uint32_t off[R::kRPT][kOffWords];  // the rows' table word offsets, two per word
+  constexpr bool kHold = C <= 4;
+  uint32_t off[R::kRPT][kOffWords];
+  auto take = [&](int j, uint64_t i) {  // offsets of row pre_row0 + i
+    if constexpr (kOffWords == 2) {
+      const uint2 v = __ldg(p.pre + i);
+      off[j][0] = v.x;
+      off[j][1] = v.y;
+    } else {
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p.pre) + i);
+      off[j][0] = v.x;
+      off[j][1] = v.y;
+      off[j][2] = v.z;
+      off[j][3] = v.w;
+    }
+  };
   auto load_offsets = [&](uint64_t b) {
     const uint64_t row0 = b * R::kRows;
     if (row0 + R::kRows <= p.nrows) {
-      const uint2 *src = p.pre + (row0 - p.pre_row0) + tid;
+      const uint64_t i = row0 - p.row_begin + tid;
 #pragma unroll
-      for (int j = 0; j < R::kRPT; j++) {
-        const uint2 v = __ldg(src + j * 256);
-        off[j][0] = v.x;
-        off[j][1] = v.y;
-      }
-    } else {
+      for (int j = 0; j < R::kRPT; j++) take(j, i + j * 256);
+    } else {  // rows past the table take its last row's offsets (their masks are zeroed)
 #pragma unroll
-      for (int j = 0; j < R::kRPT; j++) {
-        // rows past the table take its last row's offsets (their masks are zeroed)
-        const uint64_t row = min(row0 + tid + j * 256, p.nrows - 1);
-        const uint2 v = __ldg(p.pre + (row - p.pre_row0));
-        off[j][0] = v.x;
-        off[j][1] = v.y;
-      }
+      for (int j = 0; j < R::kRPT; j++) take(j, min(row0 + tid + j * 256, p.nrows - 1) - p.row_begin);
     }
   };
   auto piece = [&](int j, int s) {  // part s ^ hx of the thread's row j
     return reinterpret_cast<uint4 *>(mst + j * (256 / S * 128) + (mpos ^ (s << 4)));
   };
 
-  uint64_t blk = p.block_begin + bid;
-  if (blk < p.nblocks) load_offsets(blk);
-  for (uint32_t n = 1; blk < p.nblocks; blk += nb, n++) {
+  uint64_t blk = block_begin + bid;
+  if (kHold && blk < nblocks) load_offsets(blk);
+  for (uint32_t n = 1; blk < nblocks; blk += nb, n++) {
     const bool full = (blk + 1) * R::kRows <= p.nrows;
+    if (!kHold) load_offsets(blk);
     // ---- A ----
 #pragma unroll
     for (int j = 0; j < R::kRPT; j++) {
@@ -256,9 +257,9 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
         o[k] = __byte_perm(w[k / 2], 0u, rows_group_size(C, S, k) >= 2 ? sel[k & 1] : 0x4410u);
       if (OVF) {  // byte offsets of part hx; part s ^ hx is 16 * s away by XOR
 #pragma unroll
-        for (int k = 0; k < C; k++) o[k] = o[k] < lim[k] ? o[k] * p.t_mul[0] + lc[0][k] : o[k] * p.t_mul[1] + lo[k];
+        for (int k = 0; k < C; k++) o[k] = o[k] < lim[k] ? o[k] * L.t_mul[0] + lc[0][k] : o[k] * L.t_mul[1] + lo[k];
       }
-      auto at = [&](int k, int s) { return OVF ? o[k] ^ (s << 4) : o[k] * p.t_mul[0] + lc[OVF ? 0 : s][k]; };
+      auto at = [&](int k, int s) { return OVF ? o[k] ^ (s << 4) : o[k] * L.t_mul[0] + lc[OVF ? 0 : s][k]; };
 #pragma unroll
       for (int s = 0; s < Q; s++) {
         uint4 m = *reinterpret_cast<const uint4 *>(tables + at(0, s));
@@ -280,7 +281,15 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
 #pragma unroll
           for (int s = 0; s < Q; s++) *piece(j, s) = make_uint4(0, 0, 0, 0);
     }
-    if (blk + nb < p.nblocks) load_offsets(blk + nb);  // in flight during B and C
+    if (blk + nb < nblocks) {  // in flight during B and C
+      if (kHold) {
+        load_offsets(blk + nb);
+      } else {  // 16 bytes a row: a 128-byte line is eight rows
+        const uint64_t row = (blk + nb) * R::kRows + (uint64_t)tid * 8;
+        if (tid < R::kRows / 8 && row < p.nrows)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4 *>(p.pre) + (row - p.row_begin)));
+      }
+    }
     __syncthreads();
     // ---- B ----
     uint32_t x[32];
@@ -301,7 +310,7 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
       }
       if ((n & 1023) == 0)  // a block adds at most 32 to a 16-bit counter
         flush([&](int slot, uint32_t c) {
-          const int32_t q = (int32_t)__ldg(p.blob + p.slot_off + half * 256 + slot);
+          const int32_t q = (int32_t)__ldg(p.blob + p.slot_off + 32 * g0 + slot);
           if (q >= 0) atomicAdd(p.counts + q, (unsigned long long)c);
         });
     }
@@ -314,10 +323,10 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
         const uint32_t src = (uint32_t)__cvta_generic_to_shared(buf);
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-          const int line0 = Q == 2 ? 256 * half + 128 * i : 0;
+          const int line0 = 32 * g0 + (Q == 2 ? 128 * i : 0);
           if (line0 < (int)p.nslots)
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
-                             &tmap),
+                             tmap),
                          "r"((uint32_t)word + (Q == 2 ? 0 : 32 * i)), "r"(line0), "r"(src + 16384 * i)
                          : "memory");
         }
@@ -328,8 +337,7 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
       __syncthreads();
       const int c = lane & 7;
       for (int i = tid >> 3; i < 256; i += 32) {
-        const int slot = Q == 2 ? 256 * half + rows_slot(i) : rows_slot(i & 127);
-        const int32_t q = (int32_t)__ldg(p.blob + p.slot_off + slot);
+        const int32_t q = (int32_t)__ldg(p.blob + p.slot_off + 32 * g0 + rows_slot(Q == 2 ? i : i & 127));
         if (q < 0) continue;
         const uint4 v = *reinterpret_cast<const uint4 *>(buf + i * 128 + ((c ^ (i & 7)) << 4));
         const uint64_t w = word + (Q == 2 ? 0 : 32 * (i >> 7)) + c * 4;
@@ -353,9 +361,29 @@ __global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constan
   __syncthreads();
   if (used) flush([&](int slot, uint32_t c) { atomicAdd(&sum[slot], c); });
   __syncthreads();
-  if (tid < 32 * R::kG && sum[tid]) {
-    const int32_t q = (int32_t)__ldg(p.blob + p.slot_off + half * 256 + tid);
+  if (tid < 32 * KG && sum[tid]) {
+    const int32_t q = (int32_t)__ldg(p.blob + p.slot_off + 32 * g0 + tid);
     if (q >= 0) atomicAdd(p.counts + q, (unsigned long long)sum[tid]);
+  }
+}
+
+// A pass of up to 32 * G queries: one part of 4 or 8 groups (G = 4, 8), one of 8
+// and one of 4 (G = 12: up to 384 queries), or two of 8 (G = 16).  The first
+// p.split CTAs take the first part.
+template <int C, int G, bool OVF>
+__global__ void __launch_bounds__(256, 2) batch_rows_kernel(const __grid_constant__ BatchPass p,
+                                                            const __grid_constant__ CUtensorMap tmap) {
+  static_assert(G == 4 || G == 8 || G == 12 || G == 16, "parts of four and eight groups");
+  if (G <= 8) {
+    batch_rows_part<C, G == 4 ? 4 : 8, OVF>(p, p.lay[0], &tmap, 0, blockIdx.x, gridDim.x);
+  } else if (G == 16) {
+    const bool second = blockIdx.x >= p.split;
+    batch_rows_part<C, 8, OVF>(p, p.lay[0], &tmap, second ? 8 : 0, blockIdx.x - (second ? p.split : 0),
+                               second ? gridDim.x - p.split : p.split);
+  } else if (blockIdx.x < p.split) {
+    batch_rows_part<C, 8, OVF>(p, p.lay[0], &tmap, 0, blockIdx.x, p.split);
+  } else {
+    batch_rows_part<C, 4, OVF>(p, p.lay[1], &tmap, 8, blockIdx.x - p.split, gridDim.x - p.split);
   }
 }
 
@@ -382,11 +410,12 @@ inline bool rows_tensor_map(const BatchPass &bp, uint32_t *first, CUtensorMap *m
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Table layout of a pass of bp.ncols columns and `groups` groups in shared
-// memory: as many lines as `limit` bytes hold beside the buffer, the
+// Table layout in shared memory of a part of kg groups of a pass of `groups`
+// groups: as many lines as `limit` bytes hold beside the buffer, the
 // positions past them packed behind.
-inline void rows_layout(BatchPass &bp, int groups, size_t limit) {
-  const int kg = std::min(groups, 8), S = 32 / kg, C = bp.ncols;
+inline RowsLayout rows_layout(const BatchPass &bp, int groups, int kg, size_t limit) {
+  RowsLayout L;
+  const int S = 32 / kg, C = bp.ncols;
   const uint32_t row = 4 * kg;  // bytes of a table row
   auto bytes = [&](uint32_t lines) {
     uint64_t at = 0;
@@ -396,28 +425,30 @@ inline void rows_layout(BatchPass &bp, int groups, size_t limit) {
         uint32_t m = 0;
         for (int k = 0; k < size; k++) m = std::max(m, bp.m[c + k]);
         for (int k = 0; k < size; k++) {
-          bp.t_base[c + k] = (uint32_t)(at + k * row);
-          bp.t_rep[c + k] = size * row;
-          bp.t_nrep[c + k] = S / size;
+          L.t_base[c + k] = (uint32_t)(at + k * row);
+          L.t_rep[c + k] = size * row;
+          L.t_nrep[c + k] = S / size;
         }
         at += (uint64_t)std::min(m + 1, lines) * 128;
       }
     }
     for (int c = 0; c < C; c++) {
-      bp.t_over[c] = (uint32_t)at;
+      L.t_over[c] = (uint32_t)at;
       if (bp.m[c] + 1 > lines) at += (uint64_t)(bp.m[c] + 1 - lines) * row;
     }
     return at;
   };
+  memset(&L, 0, sizeof L);
   uint32_t lo = 0, hi = 0;  // the most lines that fit
   for (int c = 0; c < C; c++) hi = std::max(hi, bp.m[c] + 1);
-  bp.t_ovf = bytes(hi) + kRowsBuffer > limit;
-  while (bp.t_ovf && hi - lo > 1) {
+  L.t_ovf = bytes(hi) + kRowsBuffer > limit;
+  while (L.t_ovf && hi - lo > 1) {
     const uint32_t mid = (lo + hi) / 2;
     (bytes(mid) + kRowsBuffer > limit ? hi : lo) = mid;
   }
-  bp.t_lines = bp.t_ovf ? lo : hi;
-  bp.t_bytes = (uint32_t)bytes(bp.t_lines);
-  bp.t_mul[0] = 128 / groups;
-  bp.t_mul[1] = row / groups;
+  L.t_lines = L.t_ovf ? lo : hi;
+  L.t_bytes = (uint32_t)bytes(L.t_lines);
+  L.t_mul[0] = 128 / groups;
+  L.t_mul[1] = row / groups;
+  return L;
 }

@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 KINDS = [lambda n, s: D.normal(n, s), lambda n, s: D.zipf(n, s, 1.2), lambda n, s: D.uniform(n, s),
-         lambda n, s: D.uniform(n, s, 256)]
+         lambda n, s: D.uniform(n, s, 256), lambda n, s: D.uniform(n, s, 1 << 20), lambda n, s: D.zipf(n, s, 1.5),
+         lambda n, s: D.normal(n, s), lambda n, s: D.uniform(n, s, 64)]
 
 
 def check(ctx, cols, queries, pad_words):
@@ -35,23 +36,23 @@ def check(ctx, cols, queries, pad_words):
     assert (got[:, words:] == 0xFFFFFFFF).all(), "wrote past a bitmap"
 
 
-@pytest.mark.parametrize("ncols", [1, 2, 3, 4])
-@pytest.mark.parametrize("nq,n", [(21, 2047), (128, 2049), (129, 1023), (256, 1025), (257, 4128), (385, 1024),
+@pytest.mark.parametrize("ncols", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("nq,n", [(21, 2047), (128, 2049), (129, 1023), (256, 1025), (300, 4128), (385, 1024),
                                   (512, 2080)])
 def test_rows_pass_at_block_edges(ctx, ncols, nq, n):
     cols = [KINDS[c](n, 31 * n + c) for c in range(ncols)]
     ctx.load_columns(cols)
-    queries = D.batch_queries(cols, nq, seed=nq + ncols, max_cols=ncols)
+    queries = D.batch_queries(cols, nq, seed=nq + ncols, max_cols=min(ncols, 6))
     check(ctx, cols, queries, 0)
 
 
 @pytest.mark.parametrize("pad_words", [0, 1])
-@pytest.mark.parametrize("nq", [100, 200, 500])
-def test_rows_pass_many_blocks(ctx, nq, pad_words):
+@pytest.mark.parametrize("nq,ncols", [(100, 3), (200, 3), (384, 3), (500, 3), (300, 6)])
+def test_rows_pass_many_blocks(ctx, nq, ncols, pad_words):
     """More than one block per CTA, a last block that is not full, a query in
     the middle that the pass does not hold (bitmaps out of order)."""
     n = 2 * 296 * 2048 + 545
-    cols = [KINDS[c](n, 77 + c) for c in range(3)]
+    cols = [KINDS[c](n, 77 + c) for c in range(ncols)]
     ctx.load_columns(cols)
     queries = D.batch_queries(cols, nq, seed=nq)
     if pad_words:
@@ -72,3 +73,15 @@ def test_rows_pass_positions_past_the_lines(ctx):
     queries = [[(0, int(a), int(b))] + ([(1, i % 40, 50)] if i % 3 == 0 else []) for i, (a, b) in
                enumerate(zip(lo, hi))]
     check(ctx, cols, queries, 0)
+
+
+def test_passes_over_different_columns_share_in_groups(ctx):
+    """Passes over two sets of columns (the second of more than four), then
+    more passes than one group holds."""
+    n = 9_001
+    cols = [KINDS[c](n, 5 + c) for c in range(8)]
+    ctx.load_columns(cols)
+    first = D.batch_queries(cols[:2], 512, seed=1, max_cols=2)
+    second = [[(2 + c, lo, hi) for c, lo, hi in q] for q in D.batch_queries(cols[2:], 600, seed=2, max_cols=3)]
+    check(ctx, cols, first + second, 0)
+    check(ctx, cols, D.batch_queries(cols[:3], 512 * 5 + 40, seed=3, max_cols=3), 0)

@@ -1,6 +1,7 @@
 """Index arithmetic of the thread-per-row pass kernel, on the CPU.
 
-batch_rows_kernel (rtscan_b200/csrc/batch_rows.cuh) keeps a pass's tables
+batch_rows_kernel (rtscan_b200/csrc/batch_rows.cuh; a part of kg groups of a
+pass of G) keeps a pass's tables
 in 128-byte lines whose slots hold copies of the columns of a group, lets
 lane i of a quarter-warp visit the slots and 16-byte parts in the order
 k ^ i, writes the row masks to a swizzled buffer, transposes 32-row tiles of
@@ -33,10 +34,9 @@ def groups_of(C, S):
     return out
 
 
-def layout(C, G, m, lines):
+def layout(C, kg, m, lines):
     """Byte offsets as rows_layout gives them for at most `lines` lines:
     first copies, bytes between copies, copies, rows past the lines, all."""
-    kg = min(G, 8)
     S, row = 32 // kg, 4 * kg
     grp = groups_of(C, S)
     base, rep, nrep, over = [0] * C, [0] * C, [1] * C, [0] * C
@@ -81,12 +81,11 @@ def one_per_bank(addr, lanes, banks, width):
 
 
 @pytest.mark.parametrize("lines", [1 << 20, 17, 0])
-@pytest.mark.parametrize("G", [16, 8, 4])
+@pytest.mark.parametrize("G,kg", [(16, 8), (16, 4), (8, 8), (4, 4)])
 @pytest.mark.parametrize("C", [1, 2, 3, 4, 5, 6, 7, 8])
-def test_rows_kernel_addresses(C, G, lines):
+def test_rows_kernel_addresses(C, G, kg, lines):
     rng = np.random.default_rng(100 * C + G)
-    kg = min(G, 8)
-    half = G // kg - 1
+    g0 = 8 if G == 16 else 0  # the part's first group
     Q = kg // 4
     LQ = {2: 1, 1: 0}[Q]
     S, LS, RPT = 8 // Q, 3 - LQ, 32 // kg
@@ -94,7 +93,7 @@ def test_rows_kernel_addresses(C, G, lines):
     tiles = rows // 32
     m = [int(x) for x in rng.integers(0, 40, C)]
     grp = groups_of(C, S)
-    base, rep, nrep, over, total = layout(C, G, m, lines)
+    base, rep, nrep, over, total = layout(C, kg, m, lines)
     mul, mul_over = 128 // G, 4 * kg // G
     tab = [rng.integers(0, 2**32, size=(m[c] + 1, G), dtype=np.uint64) for c in range(C)]
     tab_off, at = [], 0  # word offsets in the plan blob
@@ -109,7 +108,7 @@ def test_rows_kernel_addresses(C, G, lines):
             for w in (a // 4 for a in at):
                 assert w + kg <= smem.size
                 assert np.all(smem[w:w + kg] == 2**40), "two table rows share words"
-                smem[w:w + kg] = tab[c][pos, half * kg:half * kg + kg]
+                smem[w:w + kg] = tab[c][pos, g0:g0 + kg]
 
     # phase A, all 256 threads
     tid = np.arange(256)
@@ -156,7 +155,7 @@ def test_rows_kernel_addresses(C, G, lines):
         assert one_per_bank(ld, 32, 32, 4), "mask loads of a warp share banks"
         want = np.full(256, FULL, dtype=np.uint64)
         for c in range(C):
-            want &= tab[c][pos[c][32 * tile + r], half * kg + group]
+            want &= tab[c][pos[c][32 * tile + r], g0 + group]
         assert np.array_equal(buf[ld // 4], want)
         x[:, (r & 24) | (7 - (r & 7))] = buf[ld // 4]
     x = transpose_octets(x)
@@ -171,7 +170,7 @@ def test_rows_kernel_addresses(C, G, lines):
         buf[st // 4] = x[:, j]
 
     # phase C: line i holds query i's words, its 16-byte chunk c at c ^ (i % 8)
-    mask = np.stack([np.bitwise_and.reduce([tab[c][pos[c], half * kg + g] for c in range(C)])
+    mask = np.stack([np.bitwise_and.reduce([tab[c][pos[c], g0 + g] for c in range(C)])
                      for g in range(kg)], 1)  # [row, group]
     slots = set()
     for i in range(32 * kg):
