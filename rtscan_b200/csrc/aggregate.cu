@@ -7,10 +7,10 @@
 // kernels are HBM-bound streaming passes:
 //
 //   * rts_bitmap_rows_async: ordered compaction of a bitmap into ascending
-//     uint32 row ids.  Pass 1 counts the set bits of each 4096-word tile;
-//     one CTA turns the tile counts into output offsets; pass 2 reloads each
-//     tile into shared memory and every thread expands its 16 consecutive
-//     words at its exclusive prefix.  Bytes: 2 x N/8 read + 4 per row id.
+//     uint32 row ids.  Pass 1 counts the set bits of each 1024-word tile;
+//     pass 2 reloads each tile, sums the counts before it (past 2^28 rows a
+//     one-CTA scan does) and every warp expands its words one at a time, a
+//     lane per bit.  Bytes: 2 x N/8 read + 4 per row id.
 //   * rts_bitmap_sum_async: sum of a column, or of the product of two
 //     columns, over the set rows (128-bit exact).  A warp takes 1024 rows:
 //     its 32 bitmap words, then the values as 16-byte loads, each lane
@@ -34,24 +34,35 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kCompactThreads = 256;
-constexpr int kCompactWordsPerThread = 16;
-constexpr int kCompactTileWords = kCompactThreads * kCompactWordsPerThread;  // 4096 words = 131072 rows
+constexpr int kCompactRounds = 4;                                   // words per thread
+constexpr int kCompactTileWords = kCompactThreads * kCompactRounds;  // 1024 words = 32768 rows
 constexpr int kScanThreads = 1024;
+// Up to this many tiles (2^28 rows) every block of the write pass sums the
+// counts of the tiles before it itself (at most 32 loads per thread, from
+// L2); a scan launch of one block costs about 3 us.
+constexpr uint64_t kCompactSelfTiles = 8192;
 
-// Bitmap words of tile t, padded so that thread i's 16 consecutive words sit
-// in 16 different banks from its neighbours' (index w + w/16).
-__device__ __forceinline__ int pad16(int w) { return w + (w >> 4); }
+// The thread's kCompactRounds words of the tile: warp w's round r holds words
+// 32 * (kCompactRounds * w + r) .. + 31 of it, one per lane.
+__device__ __forceinline__ void compact_words(const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask,
+                                              uint32_t (&x)[kCompactRounds]) {
+  const uint64_t w0 = (uint64_t)blockIdx.x * kCompactTileWords + (threadIdx.x >> 5) * (32 * kCompactRounds) +
+                      (threadIdx.x & 31);
+#pragma unroll
+  for (int r = 0; r < kCompactRounds; r++) {
+    const uint64_t w = w0 + 32 * r;
+    x[r] = w < words ? (w + 1 == words ? __ldg(bm + w) & tail_mask : __ldg(bm + w)) : 0u;
+  }
+}
 
 __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(const uint32_t *__restrict__ bm,
                                                                         uint64_t words, uint32_t tail_mask,
                                                                         uint32_t *__restrict__ tile_count) {
-  const uint64_t w0 = (uint64_t)blockIdx.x * kCompactTileWords;
+  uint32_t x[kCompactRounds];
+  compact_words(bm, words, tail_mask, x);
   uint32_t c = 0;
 #pragma unroll
-  for (int j = 0; j < kCompactWordsPerThread; j++) {
-    const uint64_t w = w0 + j * kCompactThreads + threadIdx.x;
-    if (w < words) c += __popc(w + 1 == words ? bm[w] & tail_mask : bm[w]);
-  }
+  for (int r = 0; r < kCompactRounds; r++) c += __popc(x[r]);
   c = __reduce_add_sync(kFull, c);
   __shared__ uint32_t part[kCompactThreads / 32];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
@@ -101,47 +112,92 @@ __global__ void __launch_bounds__(kScanThreads) compact_scan_kernel(const uint32
   if (threadIdx.x == kScanThreads - 1) *total = off;
 }
 
+// A warp expands its words one at a time: lane l holds bit l's row, so a
+// word's ids leave as one run of consecutive addresses (the pass before had
+// every thread store the ids of 16 words at its own place: 32 lines per
+// store instruction).  tile_off null: the block sums the counts before its
+// tile, and the last block stores the total.
+// Bound by issue, about 12 instructions per nonzero word (and one POPC), then
+// by the id writes.  2^25 rows, a two-column scan of 10-50 % and its row ids:
+// 127 -> 82 us a pass; of that the write pass takes 29 us and the count 3.
 __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
-    const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask,
-    const unsigned long long *__restrict__ tile_off, uint32_t *__restrict__ rows, uint64_t capacity) {
-  __shared__ uint32_t tile[kCompactTileWords + kCompactTileWords / 16];
-  __shared__ uint32_t warp_sum[kCompactThreads / 32];
-  const uint64_t w0 = (uint64_t)blockIdx.x * kCompactTileWords;
-#pragma unroll
-  for (int j = 0; j < kCompactWordsPerThread; j++) {
-    const int i = j * kCompactThreads + threadIdx.x;
-    const uint64_t w = w0 + i;
-    tile[pad16(i)] = w < words ? (w + 1 == words ? bm[w] & tail_mask : bm[w]) : 0u;
-  }
-  __syncthreads();
-  uint32_t mine[kCompactWordsPerThread];
-  uint32_t c = 0;
-#pragma unroll
-  for (int j = 0; j < kCompactWordsPerThread; j++) {
-    mine[j] = tile[pad16(threadIdx.x * kCompactWordsPerThread + j)];
-    c += __popc(mine[j]);
-  }
+    const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask, const uint32_t *__restrict__ tile_count,
+    const unsigned long long *__restrict__ tile_off, uint32_t *__restrict__ rows, uint64_t capacity,
+    unsigned long long *__restrict__ total) {
+  __shared__ unsigned long long s_before[kCompactThreads / 32];
+  __shared__ uint32_t s_warp[kCompactThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t incl = c;
+  uint32_t x[kCompactRounds];
+  compact_words(bm, words, tail_mask, x);
+  unsigned long long before = 0;
+  if (!tile_off) {
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kCompactThreads) before += __ldg(tile_count + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(kFull, before, o);
+    if (lane == 0) s_before[warp] = before;
+  }
+  // inclusive scans of the rounds' popcounts over the lanes, two rounds to a
+  // word (a round has at most 1024 bits)
+  static_assert(kCompactRounds == 4, "two packed scans");
+  uint32_t c01 = __popc(x[0]) | __popc(x[1]) << 16, c23 = __popc(x[2]) | __popc(x[3]) << 16;
+  const uint32_t own01 = c01, own23 = c23;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += y;
+    const uint32_t y01 = __shfl_up_sync(kFull, c01, o), y23 = __shfl_up_sync(kFull, c23, o);
+    if (lane >= o) {
+      c01 += y01;
+      c23 += y23;
+    }
   }
-  if (lane == 31) warp_sum[warp] = incl;
+  const uint32_t all01 = __shfl_sync(kFull, c01, 31), all23 = __shfl_sync(kFull, c23, 31);
+  c01 -= own01;
+  c23 -= own23;
+  const uint32_t sum[kCompactRounds] = {all01 & 0xFFFFu, all01 >> 16, all23 & 0xFFFFu, all23 >> 16};
+  if (lane == 0) s_warp[warp] = sum[0] + sum[1] + sum[2] + sum[3];
   __syncthreads();
-  uint32_t before = 0;
-  for (int k = 0; k < warp; k++) before += warp_sum[k];
-  unsigned long long o = tile_off[blockIdx.x] + before + incl - c;
-  const uint64_t row0 = (w0 + (uint64_t)threadIdx.x * kCompactWordsPerThread) * 32;
+  uint32_t start = 0, tile = 0;  // ids of the tile before this warp, in the tile
 #pragma unroll
-  for (int j = 0; j < kCompactWordsPerThread; j++) {
-    uint32_t w = mine[j];
-    while (w) {  // MSB-first: bit 31 is the word's first row
-      const int b = __clz(w);
-      if (o < capacity) rows[o] = (uint32_t)(row0 + j * 32 + b);
-      o++;
-      w &= ~(0x80000000u >> b);
+  for (int k = 0; k < kCompactThreads / 32; k++) {
+    if (k < warp) start += s_warp[k];
+    tile += s_warp[k];
+  }
+  unsigned long long base = 0;
+  if (tile_off) {
+    base = tile_off[blockIdx.x];
+  } else {
+#pragma unroll
+    for (int k = 0; k < kCompactThreads / 32; k++) base += s_before[k];
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = base + tile;
+  }
+  if (base >= capacity) return;
+  // the warp's nonzero words, each with its index and its ids' offset in the tile
+  __shared__ uint2 s_word[kCompactThreads / 32][32 * kCompactRounds];
+  uint2 *const list = s_word[warp];
+  int n = 0;
+#pragma unroll
+  for (int r = 0; r < kCompactRounds; r++) {
+    const uint32_t off = start + (r == 0 ? c01 & 0xFFFFu : r == 1 ? c01 >> 16 : r == 2 ? c23 & 0xFFFFu : c23 >> 16);
+    const unsigned some = __ballot_sync(kFull, x[r] != 0);
+    if (x[r]) list[n + __popc(some & ((1u << lane) - 1))] = make_uint2(x[r], off | (uint32_t)(32 * r + lane) << 16);
+    n += __popc(some);
+    start += sum[r];
+  }
+  __syncwarp();
+  uint32_t *const dst = rows + base;
+  const uint32_t row = (uint32_t)(((uint64_t)blockIdx.x * kCompactTileWords + warp * (32 * kCompactRounds)) * 32) + lane;
+  const uint32_t bit = 0x80000000u >> lane, above = ~(0xFFFFFFFFu >> lane);  // MSB-first: bit 31 is the word's first row
+  const uint32_t room = (uint32_t)std::min<unsigned long long>(capacity - base, 0xFFFFFFFFull);
+  if (room >= tile) {
+#pragma unroll 4
+    for (int k = 0; k < n; k++) {
+      const uint2 w = list[k];
+      if (w.x & bit) dst[(w.y & 0xFFFFu) + __popc(w.x & above)] = row + ((w.y >> 16) << 5);
+    }
+  } else {
+    for (int k = 0; k < n; k++) {
+      const uint2 w = list[k];
+      const uint32_t at = (w.y & 0xFFFFu) + __popc(w.x & above);
+      if ((w.x & bit) && at < room) dst[at] = row + ((w.y >> 16) << 5);
     }
   }
 }
@@ -352,17 +408,18 @@ rts_status rts_bitmap_rows_async(rts_ctx *ctx, const uint32_t *dev_bitmap, uint6
     }
     const uint32_t tail_mask = (nrows & 31) ? ~(0xFFFFFFFFu >> (nrows & 31)) : 0xFFFFFFFFu;
     const uint64_t ntiles = (words + rts::kCompactTileWords - 1) / rts::kCompactTileWords;
+    const bool self = ntiles <= rts::kCompactSelfTiles;
     char *scratch = static_cast<char *>(rts::agg_scratch(ctx, ntiles * 12 + 16));
-    auto *tile_off = reinterpret_cast<unsigned long long *>(scratch);
+    auto *tile_off = self ? nullptr : reinterpret_cast<unsigned long long *>(scratch);
     auto *tile_count = reinterpret_cast<uint32_t *>(scratch + ntiles * 8);
+    auto *total = reinterpret_cast<unsigned long long *>(dev_count);
     rts::compact_count_kernel<<<(unsigned)ntiles, rts::kCompactThreads, 0, s>>>(dev_bitmap, words, tail_mask,
                                                                                tile_count);
-    rts::compact_scan_kernel<<<1, rts::kScanThreads, 0, s>>>(tile_count, ntiles, tile_off,
-                                                             reinterpret_cast<unsigned long long *>(dev_count));
-    rts::compact_write_kernel<<<(unsigned)ntiles, rts::kCompactThreads, 0, s>>>(dev_bitmap, words, tail_mask,
-                                                                               tile_off, dev_rows, capacity);
+    if (!self) rts::compact_scan_kernel<<<1, rts::kScanThreads, 0, s>>>(tile_count, ntiles, tile_off, total);
+    rts::compact_write_kernel<<<(unsigned)ntiles, rts::kCompactThreads, 0, s>>>(
+        dev_bitmap, words, tail_mask, tile_count, tile_off, dev_rows, capacity, total);
     RTS_CUDA(cudaGetLastError());
-    ctx->launches += 3;
+    ctx->launches += self ? 2 : 3;
     return RTS_OK;
   } catch (const std::exception &e) {
     return rts::fail(ctx, e);
