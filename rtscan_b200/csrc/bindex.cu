@@ -111,7 +111,9 @@ __global__ void area_kernel(const uint32_t *sval, uint64_t n, int K, uint32_t *s
   }
 }
 
+// out[j] = sval[j * stride], j < m; out[m] = the last value.
 __global__ void sample_kernel(const uint32_t *sval, uint64_t n, uint32_t *out, uint64_t m, uint64_t stride) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) out[m] = sval[n - 1];
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m; j += (uint64_t)gridDim.x * blockDim.x)
     out[j] = sval[j * stride];
 }
@@ -542,9 +544,38 @@ int blocks_for(uint64_t items, int sm_count, int per_sm) {
 }  // namespace
 
 GpuBinDex::~GpuBinDex() {
-  if (sval) cudaFree(sval);
-  if (spos) cudaFree(spos);
-  if (fv) cudaFree(fv);
+  if (base) cudaFree(base);
+}
+
+uint32_t *GpuBinDex::allocate(uint64_t rows, int areas, std::unique_ptr<GpuBinDex> old) {
+  n = rows;
+  K = areas;
+  fv_stride = (((n + 31) >> 5) + 3) / 4 * 4;
+  // 256-byte aligned arrays, those of 32 MiB and more at 2 MiB pages (a query
+  // of two columns at 1e8 rows took 1 % longer without)
+  auto padded = [](uint64_t words) {
+    const uint64_t to = words >= (1u << 23) ? 1u << 19 : 64;
+    return (words + to - 1) / to * to;
+  };
+  const uint64_t col_words = padded(n), fv_words = padded((uint64_t)(K - 1) * fv_stride);
+  const size_t bytes = (2 * col_words + fv_words + padded(bindex_table_words(n, K))) * 4;
+  if (old && old->cap >= bytes && old->cap <= 2 * bytes) {
+    RTS_CUDA(cudaDeviceSynchronize());  // queries that still read the old index, on any stream
+    std::swap(base, old->base);
+    cap = old->cap;
+  } else {
+    old.reset();
+    if (cudaMalloc(&base, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      base = nullptr;
+      throw Error(RTS_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed");
+    }
+    cap = bytes;
+  }
+  sval = static_cast<uint32_t *>(base);
+  spos = sval + col_words;
+  fv = spos + col_words;
+  return fv + fv_words;
 }
 
 namespace {
@@ -576,24 +607,28 @@ uint64_t count_fv_mismatches(const uint32_t *col, uint64_t n, const uint32_t *d_
   return bad;
 }
 
-std::unique_ptr<GpuBinDex> build_bindex(const uint32_t *col, uint64_t n, int K, int sm_count, cudaStream_t s) {
+std::unique_ptr<GpuBinDex> build_bindex(const uint32_t *col, uint64_t n, int K, int sm_count, cudaStream_t s,
+                                        std::unique_ptr<GpuBinDex> old) {
   if (K < 2 || K > 4096) throw Error(RTS_ERR_ARG, "K must be in [2, 4096]");
   if (n < (uint64_t)K) throw Error(RTS_ERR_ARG, "BinDex needs at least K rows");
   if (n >= (1ull << 32)) throw Error(RTS_ERR_ARG, "BinDex supports fewer than 2^32 rows per column");
   auto b = std::make_unique<GpuBinDex>();
-  b->K = K;
-  b->n = n;
-  b->sval = dev_alloc<uint32_t>(n);
-  b->spos = dev_alloc<uint32_t>(n);
-  uint32_t *ids = dev_alloc<uint32_t>(n);
-  DevFree f_ids{ids};
+  uint32_t *tables = b->allocate(n, K, std::move(old));
+  // row ids and sort scratch: in the filter vectors' place, which are written
+  // after the sort, when they fit (K >= 98 or so), else for the call
   size_t temp_bytes = 0;
-  RTS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, col, b->sval, ids, b->spos, (int64_t)n, 0, 32, s));
-  void *temp = dev_alloc<char>(temp_bytes);
-  DevFree f_temp{temp};
+  RTS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, col, b->sval, b->spos, b->spos, (int64_t)n, 0, 32, s));
+  const uint64_t ids_words = (n + 63) / 64 * 64, fv_words = (uint64_t)(K - 1) * b->fv_stride;
+  DevFree f_temp{nullptr};
+  uint32_t *ids = b->fv;
+  if (ids_words * 4 + temp_bytes > fv_words * 4) {
+    ids = dev_alloc<uint32_t>(ids_words + (temp_bytes + 3) / 4);
+    f_temp.p = ids;
+  }
+  void *temp = ids + ids_words;
   // Sorted by the bits in use only: a column of 20-bit codes takes three
   // passes of eight bits instead of four (2^25 rows: 640 instead of 810 us).
-  uint32_t *d_bits = static_cast<uint32_t *>(temp), bits = 0;  // (free until the sort)
+  uint32_t *d_bits = tables, bits = 0;
   RTS_CUDA(cudaMemsetAsync(d_bits, 0, 4, s));
   iota_bits_kernel<<<blocks_for(n / 4 + 1, sm_count, 8), kThreads, 0, s>>>(col, n, ids, ((uintptr_t)col & 15) == 0,
                                                                            d_bits);
@@ -606,35 +641,23 @@ std::unique_ptr<GpuBinDex> build_bindex(const uint32_t *col, uint64_t n, int K, 
   if (need > temp_bytes) end_bit = 32;
   RTS_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, col, b->sval, ids, b->spos, (int64_t)n, 0, end_bit, s));
 
-  uint32_t *d_start = dev_alloc<uint32_t>(K);
-  DevFree f_start{d_start};
-  unsigned long long *d_rank = dev_alloc<unsigned long long>(K);
-  DevFree f_rank{d_rank};
-  area_kernel<<<(K * 32 + kThreads - 1) / kThreads, kThreads, 0, s>>>(b->sval, n, K, d_start, d_rank);
+  // the tables: area ranks, start values, the sample and the last value
   const uint64_t m = (n + kSampleStride - 1) / kSampleStride;
-  uint32_t *d_sample = dev_alloc<uint32_t>(m);
-  DevFree f_sample{d_sample};
+  unsigned long long *d_rank = reinterpret_cast<unsigned long long *>(tables);
+  uint32_t *d_start = tables + 2 * (uint64_t)K, *d_sample = d_start + K;
+  area_kernel<<<(K * 32 + kThreads - 1) / kThreads, kThreads, 0, s>>>(b->sval, n, K, d_start, d_rank);
   sample_kernel<<<blocks_for(m, sm_count, 4), kThreads, 0, s>>>(b->sval, n, d_sample, m, kSampleStride);
-
-  b->fv_stride = (((n + 31) >> 5) + 3) / 4 * 4;
-  if (K > 1) {
-    b->fv = dev_alloc<uint32_t>((size_t)(K - 1) * b->fv_stride);
-    launch_fv<false>(col, n, d_start, K, b->fv, b->fv_stride, nullptr, sm_count, s);
-  }
+  launch_fv<false>(col, n, d_start, K, b->fv, b->fv_stride, nullptr, sm_count, s);
   RTS_CUDA(cudaGetLastError());
-  b->start.resize(K);
-  std::vector<unsigned long long> rk(K);
-  b->sample.resize(m);
-  RTS_CUDA(cudaMemcpyAsync(b->start.data(), d_start, K * 4, cudaMemcpyDeviceToHost, s));
-  RTS_CUDA(cudaMemcpyAsync(rk.data(), d_rank, K * 8, cudaMemcpyDeviceToHost, s));
-  RTS_CUDA(cudaMemcpyAsync(b->sample.data(), d_sample, m * 4, cudaMemcpyDeviceToHost, s));
-  uint32_t ends[2];
-  RTS_CUDA(cudaMemcpyAsync(&ends[0], b->sval, 4, cudaMemcpyDeviceToHost, s));
-  RTS_CUDA(cudaMemcpyAsync(&ends[1], b->sval + n - 1, 4, cudaMemcpyDeviceToHost, s));
+  std::vector<uint32_t> host(bindex_table_words(n, K));
+  RTS_CUDA(cudaMemcpyAsync(host.data(), tables, host.size() * 4, cudaMemcpyDeviceToHost, s));
   RTS_CUDA(cudaStreamSynchronize(s));
-  b->first_rank.assign(rk.begin(), rk.end());
-  b->min_val = ends[0];
-  b->max_val = ends[1];
+  b->first_rank.resize(K);
+  memcpy(b->first_rank.data(), host.data(), (size_t)K * 8);
+  b->start.assign(host.begin() + 2 * K, host.begin() + 3 * K);
+  b->sample.assign(host.begin() + 3 * K, host.begin() + 3 * K + m);
+  b->min_val = host[3 * (size_t)K];
+  b->max_val = host.back();
   return b;
 }
 
@@ -930,8 +953,8 @@ rts_status rts_build_bindex(rts_ctx *ctx, int32_t column, int32_t K) {
     if (column < 0 || column >= (int)ctx->cols.size()) throw rts::Error(RTS_ERR_ARG, "column out of range");
     rts::DeviceGuard device_guard(ctx->device);
     if (ctx->bindex.size() < ctx->cols.size()) ctx->bindex.resize(ctx->cols.size());
-    ctx->bindex[column].reset();
-    auto b = rts::build_bindex(ctx->cols[column], ctx->nrows, K, ctx->sm_count, nullptr);
+    auto b = rts::build_bindex(ctx->cols[column], ctx->nrows, K, ctx->sm_count, nullptr,
+                               std::move(ctx->bindex[column]));
     ctx->launches += 5;
     ctx->bindex[column] = std::move(b);
     return RTS_OK;

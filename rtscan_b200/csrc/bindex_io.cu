@@ -284,9 +284,6 @@ rts_status rts_load_bindex(rts_ctx *ctx, int32_t column, const char *path) {
       throw rts::Error(RTS_ERR_PARSE, p + ": bad sample count");
     rts::DeviceGuard device_guard(ctx->device);
     auto b = std::make_unique<rts::GpuBinDex>();
-    b->K = (int)h.K;
-    b->n = h.n;
-    b->fv_stride = h.fv_stride;
     b->min_val = h.min_val;
     b->max_val = h.max_val;
     b->start.resize(h.K);
@@ -306,9 +303,7 @@ rts_status rts_load_bindex(rts_ctx *ctx, int32_t column, const char *path) {
         throw rts::Error(RTS_ERR_NOMEM, "device allocation failed");
       }
     };
-    alloc(b->sval, h.n);
-    alloc(b->spos, h.n);
-    alloc(b->fv, (uint64_t)(h.K - 1) * h.fv_stride);
+    b->allocate(h.n, (int)h.K, nullptr);  // (the column's index stays until this one is checked)
     rts::Pinned stage;
     RTS_CUDA(cudaMallocHost(&stage.p, rts::kStage));
     rts::read_device(f.f, b->sval, h.n, stage.p, p);

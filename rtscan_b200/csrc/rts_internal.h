@@ -139,6 +139,13 @@ struct GpuBinDex {
   std::vector<uint64_t> first_rank; // lower_bound of start[k] in sorted order (K), host copy
   std::vector<uint32_t> sample;     // every kSampleStride-th sorted value, host copy
   uint32_t min_val = 0, max_val = 0;
+  void *base = nullptr;  // one allocation holds sval, spos, fv and the build's tables
+  size_t cap = 0;        // its bytes
+  // Room for an index of n rows and K areas (fields n, K, fv_stride, sval,
+  // spos, fv are set), in `old`'s allocation when that is large enough and at
+  // most twice as large (one device allocation costs 0.4-2 ms here), else a
+  // new one; returns the tables (bindex_table_words() words, 8-byte aligned).
+  uint32_t *allocate(uint64_t n, int K, std::unique_ptr<GpuBinDex> old);
   ~GpuBinDex();
 };
 constexpr int kSampleStride = 1024;
@@ -149,8 +156,15 @@ constexpr int kQuerySlots = 64;
 // give for the column: 0 for a consistent index.  Synchronises stream s.
 uint64_t count_fv_mismatches(const uint32_t *col, uint64_t n, const uint32_t *d_start, int K, const uint32_t *fv,
                              uint64_t fv_stride, unsigned long long *d_bad, int sm_count, cudaStream_t s);
-std::unique_ptr<GpuBinDex> build_bindex(const uint32_t *col, uint64_t n, int K, int sm_count,
-                                        cudaStream_t s);
+// Words of the build's tables: area ranks (two each) and start values,
+// every kSampleStride-th sorted value, and the last one.
+inline uint64_t bindex_table_words(uint64_t n, int K) {
+  return 3 * (uint64_t)K + (n + kSampleStride - 1) / kSampleStride + 1;
+}
+// Builds the index of a column; `old` (may be null) is an index that it
+// replaces, whose memory it may take over.
+std::unique_ptr<GpuBinDex> build_bindex(const uint32_t *col, uint64_t n, int K, int sm_count, cudaStream_t s,
+                                        std::unique_ptr<GpuBinDex> old);
 // Conjunctive query through the column indexes (all referenced columns
 // must be indexed).  Throws rts::Error.
 void bindex_query(rts_ctx *ctx, const rts_term *terms, int nterms, uint32_t *out, unsigned long long *count,
