@@ -120,9 +120,10 @@ void fused(rts_ctx *ctx, const Plan &plan, uint32_t *out, unsigned long long *co
     check_launch(ctx, 1);
     return;
   }
-  if (count) RTS_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), s));
   const size_t T = plan.terms.size();
   int launches = 0;
+  const bool one = count && T <= (size_t)rts::kFusedMaxTerms;  // (several launches AND into the bitmap)
+  if (count && !one) RTS_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), s));
   for (size_t first = 0; first < T; first += rts::kFusedMaxTerms) {
     rts::ScanParams p;
     memset(&p, 0, sizeof p);
@@ -138,7 +139,10 @@ void fused(rts_ctx *ctx, const Plan &plan, uint32_t *out, unsigned long long *co
     p.count = (first + cnt == T) ? count : nullptr;
     p.nrows = n;
     p.full_tiles = n / rts::kTileRows;
-    rts::launch_scan_fused(p, vec, ctx->sm_count, s);
+    if (!one || !rts::launch_scan_small(p, vec, s)) {
+      if (one) RTS_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), s));
+      rts::launch_scan_fused(p, vec, s);
+    }
     launches++;
   }
   check_launch(ctx, launches);
@@ -414,7 +418,7 @@ rts_status rts_scan_separate_async(rts_ctx *ctx, const rts_term *terms, int32_t 
       p.out = i == 0 ? dev_bitmap : scratch_bitmap(ctx, 0);
       p.nrows = n;
       p.full_tiles = n / rts::kTileRows;
-      rts::launch_scan_fused(p, aligned16(p.t[0].col), ctx->sm_count, s);
+      rts::launch_scan_fused(p, aligned16(p.t[0].col), s);
       launches++;
       if (i > 0) {
         rts::launch_bitmap_op(RTS_BM_AND, dev_bitmap, dev_bitmap, p.out, words, 0, ctx->sm_count, s);

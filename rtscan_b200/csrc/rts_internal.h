@@ -110,7 +110,10 @@ struct LaunchShape {
   int blocks;
   int threads;
 };
-void launch_scan_fused(const ScanParams &p, bool vector_ok, int sm_count, cudaStream_t s);
+void launch_scan_fused(const ScanParams &p, bool vector_ok, cudaStream_t s);  // adds to *p.count
+// A small table's scan whose count is stored, not added (nothing zeroes it
+// before); false, with nothing launched, when the table is not small.
+bool launch_scan_small(const ScanParams &p, bool vector_ok, cudaStream_t s);
 void launch_bitmap_op(int op, uint32_t *dst, const uint32_t *a, const uint32_t *b, uint64_t words,
                       uint32_t value, int sm_count, cudaStream_t s);
 void launch_bitmap_count(const uint32_t *bm, uint64_t nbits, unsigned long long *count, int sm_count,
