@@ -1874,11 +1874,15 @@ extern "C" rts_status rts_scan_batch_host(rts_ctx *ctx, const uint32_t *const *h
     // the download of chunk r-1's words of every bitmap (one 2D copy) run
     // while chunk r is scanned, so the column upload hides under the bitmap
     // download.  Chunks are multiples of 4096 rows (the largest kernel block).
-    // Chunks of about 2^22 rows (at most 32): the first download starts
-    // after one chunk's upload and scan.  Each chunk's upload is queued with
+    // Chunks of about 2^22 rows (at most 32), below 2^25 rows of about 2^20 (at
+    // most 8): the first download starts after one chunk's upload and scan,
+    // and what follows the last upload is one chunk's scan, packing and
+    // download (48 queries on 2^23 rows x 2 columns: two chunks 2.85 ms,
+    // eight 2.57, sixteen 2.55).  Each chunk's upload is queued with
     // its scan (queueing every upload first measured 21 ms slower per 1e8 x 4
     // call: the downloads then share the link with 1.6 GB of uploads).
-    const uint64_t want_chunks = std::max<uint64_t>(1, std::min<uint64_t>(32, nrows >> 22));
+    const uint64_t want_chunks = std::max<uint64_t>(
+        1, nrows >= (1u << 25) ? std::min<uint64_t>(32, nrows >> 22) : std::min<uint64_t>(8, nrows >> 20));
     const uint64_t chunk_rows = ((nrows + want_chunks - 1) / want_chunks + 4095) / 4096 * 4096;
     const int nchunks = (int)((nrows + chunk_rows - 1) / chunk_rows);
     // events per chunk: upload, scan, counts on the host, pack, packed words on the host
@@ -1991,7 +1995,7 @@ extern "C" rts_status rts_scan_batch_host(rts_ctx *ctx, const uint32_t *const *h
       RTS_CUDA(cudaMemcpyAsync(qod, qoh, np * sizeof(uint64_t), cudaMemcpyHostToDevice, H.compute));
       H.last_h2d += (uint64_t)np * (sizeof(int32_t) + sizeof(uint64_t));
       if (r >= 2) RTS_CUDA(cudaStreamWaitEvent(H.compute, ev(r - 2, 4), 0));  // the device slot's last copy
-      rts::pack_kernel<<<np, rts::kPackThreads, 0, H.compute>>>(H.bitmaps, stride_words, w0, w1, qld, qod,
+      rts::pack_kernel<<<np * rts::kSparseCtas, rts::kPackThreads, 0, H.compute>>>(H.bitmaps, stride_words, w0, w1, qld, qod,
                                                                H.packed[ds]);
       ctx->launches++;
       RTS_CUDA(cudaEventRecord(ev(r, 3), H.compute));
@@ -2029,7 +2033,7 @@ extern "C" rts_status rts_scan_batch_host(rts_ctx *ctx, const uint32_t *const *h
       RTS_CUDA(cudaStreamWaitEvent(H.copy, ev(r, 1), 0));
       const uint64_t w0 = r0 / 32, w1 = r1 == nrows ? words : r1 / 32;
       if (sparse && w1 - w0 >= rts::kSparseMinWords) {
-        rts::nnz_kernel<<<nq, rts::kSparseThreads, 0, H.compute>>>(H.bitmaps, stride_words, w0, w1,
+        rts::nnz_kernel<<<nq * rts::kSparseCtas, rts::kSparseThreads, 0, H.compute>>>(H.bitmaps, stride_words, w0, w1,
                                                                    H.nnz + (size_t)nq * r);
         ctx->launches++;
         RTS_CUDA(cudaMemcpyAsync(H.nnz_host + (size_t)nq * r, H.nnz + (size_t)nq * r, (size_t)nq * 4,
