@@ -101,6 +101,7 @@ struct BatchPass {
   uint32_t groups;
   uint32_t split;               // CTAs of the first part
   uint32_t nslots;              // queries of the pass
+  uint32_t nbuf;                // buffers of a CTA: 2 where they fit (one part only), else 1
   int first_bitmap;             // >= 0: query i of the pass writes bitmap first_bitmap + i
   int tma;                      // the result lines leave by TMA
   uint32_t cnt_mul[2];          // 1 and 65536, passed at run time (see batch_rows_part)
@@ -617,7 +618,7 @@ template <int C, int G, bool OVF>
 void launch_rows_shape(BatchPass &bp, const CUtensorMap &map, int sm_count, cudaStream_t s) {
   static std::atomic<uint64_t> raised{0};
   raise_smem_limit(batch_rows_kernel<C, G, OVF>, raised, 227 * 1024);
-  const size_t sm = kRowsBuffer + std::max(bp.lay[0].t_bytes, bp.lay[1].t_bytes);
+  const size_t sm = bp.nbuf * kRowsBuffer + std::max(bp.lay[0].t_bytes, bp.lay[1].t_bytes);
   if (sm > 227 * 1024) throw Error(RTS_ERR_ARG, "batch pass exceeds shared memory");
   int per = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_rows_kernel<C, G, OVF>, 256, sm) != cudaSuccess ||
@@ -668,6 +669,7 @@ void launch_rows(BatchPass &bp, int sm_count, cudaStream_t s) {
   memset(bp.lay, 0, sizeof bp.lay);
   bp.lay[0] = rows_layout(bp, groups, std::min(groups, 8), kRowsHalfSM);
   if (twelve) bp.lay[1] = rows_layout(bp, groups, 4, kRowsHalfSM);
+  bp.nbuf = groups <= 8 && 2 * kRowsBuffer + bp.lay[0].t_bytes <= kRowsHalfSM ? 2 : 1;
   bp.cnt_mul[0] = 1;
   bp.cnt_mul[1] = 65536;
   CUtensorMap map;
