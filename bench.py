@@ -135,9 +135,9 @@ def host_info():
 # 8 B per row and pass (16 B) that the passes read back, traffic above the
 # algorithmic bytes by design.
 NCU_TRAFFIC = {
-    "batched": {"kernels": "pre_kernel<4,1> + 2 x batch4_kernel<4,16,16,true>",
+    "batched": {"kernels": "pre_kernel<4,1> + 2 x batch_rows_kernel<4,16,*>",
                 "capture": "2e7 rows x 4 columns, 1024 queries: the three launches of one step",
-                "bytes": (320.09e6 + 275.12e6) + (160.21e6 + 1221.65e6) + (160.61e6 + 1223.99e6),
+                "bytes": (320.10e6 + 273.14e6) + (280.35e6 + 1223.84e6) + (284.92e6 + 1222.51e6),
                 "step_bytes": 4 * 4 * 2e7 + 1024 * 2e7 / 8},
     "single": {"kernels": "scan_fused_kernel<1,1>", "capture": "1e8 rows x 1 column, one launch",
                "bytes": 408.9e6, "step_bytes": 4 * 1e8 + 1e8 / 8},

@@ -1095,16 +1095,14 @@ void move_column(BatchPass &dst, int c, const BatchPass &src, int s) {
   dst.nbk[c] = src.nbk[s];
 }
 
-// Shared positions for a plan with one or more table passes of the
-// look-ahead shapes (256 or 512 slots, at most four columns) over the same
-// columns (one pass too: on 1e8 rows x 4 columns the pre-pass and a pass
-// reading positions took 2.08 ms for 256 queries and 3.44 ms for 512,
-// against 2.67 and 3.98 ms for the pass that searches): the later passes' columns are put in the first one's order; per
+// Shared positions of table passes over the same columns (one pass too: on
+// 1e8 rows x 4 columns the pre-pass and a pass reading positions took 1.66 ms
+// for 256 queries and 2.88 ms for 512, a pass that searches its own 2.67 and
+// 3.98 ms): the later passes' columns are put in the first one's order; per
 // column the union of the passes' boundaries with its bucket index, and
 // the map from a union position to every pass's table word offset (a
 // pass's boundaries are a subset of the union, so the pass position of
-// union position k is the number of its boundaries <= B_u[k-1]).  Appended
-// to the plan blob; other plans are left as they are.
+// union position k is the number of its boundaries <= B_u[k-1]).
 // Passes `which` (the same columns each) share: fills P and appends the union
 // data to the plan blob; false (the plan unchanged) when it does not fit.
 bool share_group(BatchPlan &plan, const std::vector<int> &which, PreParams &P, size_t *off) {

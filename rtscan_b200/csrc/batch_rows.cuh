@@ -2,9 +2,9 @@
 // anonymous namespace; uses BatchPass and kFull from there).
 //
 // A pass has G groups of 32 query slots (16, 8 or 4).  A CTA of 8 warps
-// answers up to 8 of them (a 512-slot pass is two halves, each with half the
-// CTAs) on blocks of 1024 rows (2048 for 128 slots), two CTAs per SM, in
-// three phases over a 32 KiB buffer:
+// answers a part of eight or four of them (see batch_rows_kernel) on blocks of
+// 1024 rows (2048 for four groups), two CTAs per SM, in three phases over a
+// 32 KiB buffer:
 //   A. every thread ANDs the table rows of its rows, 16 bytes (four groups)
 //      at a time, and writes the row masks to the buffer;
 //   B. lane (tile, group) reads the 32 mask words of a 32-row tile for one
@@ -29,8 +29,7 @@
 //     order k ^ i, so its eight lanes are always in eight different 16-byte
 //     parts of a line, whatever their positions are;
 //   * the buffer's 16-byte pieces are swizzled by row and tile so that phase
-//     A's 16-byte stores, phase B's 4-byte loads and stores and phase C's
-//     16-byte loads meet 32 banks.
+//     A's 16-byte stores and phase B's 4-byte loads and stores meet 32 banks.
 // A table position past the lines that fit (L.t_lines) has its row packed
 // behind them instead, once: correct, with bank conflicts.  Two CTAs per SM
 // hold about 648 lines each, so a column of a 512-slot pass that every
@@ -38,8 +37,9 @@
 // Measured on 1e8 rows x 4 skewed columns, reading shared positions (the
 // kernel before it had each lane AND 16 rows for two groups and stage 16-bit
 // halves of the result words): 2.90 -> 2.35 ms for a 512-query pass, 1024
-// queries with their pre-pass 6.43 -> 5.35 ms; 250 queries 2.09 -> 1.74 ms,
-// 120 queries 1.46 -> 1.13 ms.  At 2.1e7 rows a 448-query pass keeps the
+// queries with their pre-pass 6.43 -> 5.35 ms; 250 queries 2.09 -> 1.66 ms,
+// 120 queries 1.46 -> 1.08 ms; 300 queries over 8 columns on 2^24 rows
+// (searching their own positions before) 1.18 -> 0.65 ms.  At 2.1e7 rows a 448-query pass keeps the
 // shared-memory pipe 58 % busy with 3.9 wavefronts per row (6.0 before) and
 // issues 10.9 warp instructions per row (16.0 before).  The lines stored by
 // 16-byte stores of eight lanes instead of TMA: 2.65 ms per 512-query pass;
