@@ -73,8 +73,10 @@ typedef struct rts_server rts_server;
 
 /* ---- errors and library info ------------------------------------------- */
 
-/* Message of the last failed call on `ctx`, or of the calling thread's last
- * failed context-free call when ctx is NULL.  Never NULL. */
+/* Message of the last failed call on `ctx` (of any thread's, a server's calls
+ * among them; the text stays as it is until the calling thread asks for this
+ * context's again), or of the calling thread's last failed call when ctx is
+ * NULL.  Never NULL. */
 RTS_API const char *rts_last_error(const rts_ctx *ctx);
 /* Library version string, e.g. "rtscan_b200 0.1 sm_100a". */
 RTS_API const char *rts_version(void);

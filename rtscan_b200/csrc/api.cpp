@@ -12,6 +12,7 @@
 #include <cstdint>
 #include <new>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "rts_internal.h"
@@ -197,8 +198,17 @@ rts_ctx::~rts_ctx() {
 extern "C" {
 
 const char *rts_last_error(const rts_ctx *ctx) {
-  if (ctx) return ctx->err.c_str();
-  return g_err.c_str();
+  if (!ctx) return g_err.c_str();
+  // the thread's own copy: another thread's failing server call may replace
+  // the context's message at any time
+  thread_local std::unordered_map<const rts_ctx *, std::string> copies;
+  try {
+    std::string &m = copies[ctx];
+    m = ctx->err.get();
+    return m.c_str();
+  } catch (const std::exception &) {
+    return "out of memory";
+  }
 }
 
 const char *rts_version(void) { return "rtscan_b200 0.1 sm_100a"; }

@@ -971,7 +971,7 @@ rts_status rts_drop_bindex(rts_ctx *ctx, int32_t column) {
   if (!ctx) return rts::set_thread_error(RTS_ERR_ARG, "null context");
   if (column < 0 || column >= (int)ctx->bindex.size()) {
     ctx->err = "column out of range";
-    return rts::set_thread_error(RTS_ERR_ARG, ctx->err);
+    return rts::set_thread_error(RTS_ERR_ARG, "column out of range");
   }
   ctx->bindex[column].reset();
   return RTS_OK;

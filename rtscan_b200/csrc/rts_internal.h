@@ -82,6 +82,25 @@ inline rts_status status_of(const std::exception &e) {
   return RTS_ERR_STATE;
 }
 
+// A context's last error message.  Server calls of any thread set it, some of
+// them under no lock of the server's, so it has a lock of its own.
+class LastError {
+ public:
+  LastError &operator=(const std::string &msg) {
+    std::lock_guard<std::mutex> lk(mu_);
+    msg_ = msg;
+    return *this;
+  }
+  std::string get() const {
+    std::lock_guard<std::mutex> lk(mu_);
+    return msg_;
+  }
+
+ private:
+  mutable std::mutex mu_;
+  std::string msg_;
+};
+
 // Record `msg` as the calling thread's last error (rts_last_error(NULL)).
 rts_status set_thread_error(rts_status code, const std::string &msg);
 
@@ -234,6 +253,6 @@ struct rts_ctx {
   std::string tune_report;  // JSON of the last rts_autotune_batch (rts_autotune_report)
   std::unique_ptr<rts::EncodeMap> encode;  // set by rts_encode_table
   std::atomic<uint64_t> launches{0};
-  std::string err;
+  rts::LastError err;
   ~rts_ctx();
 };

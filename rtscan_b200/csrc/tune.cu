@@ -114,9 +114,10 @@ extern "C" {
 rts_status rts_set_batch_config(rts_ctx *ctx, const rts_batch_config *cfg) {
   if (!ctx || !cfg) return rts::set_thread_error(RTS_ERR_ARG, "null argument");
   if (!valid(*cfg)) {
-    ctx->err = "batch config out of range (variant 3|4, warps 8|16, queries per pass and table budget within "
-               "the variant's limits)";
-    return rts::set_thread_error(RTS_ERR_ARG, ctx->err);
+    const char *const what = "batch config out of range (variant 3|4, warps 8|16, queries per pass and table budget "
+                             "within the variant's limits)";
+    ctx->err = what;
+    return rts::set_thread_error(RTS_ERR_ARG, what);
   }
   ctx->batch_cfg.variant = cfg->variant;
   ctx->batch_cfg.warps_per_cta = cfg->warps_per_cta;
