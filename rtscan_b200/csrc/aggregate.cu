@@ -295,9 +295,8 @@ struct AggParams {
 // 3: sum of slot 0 squared.
 // Row groups (four rows) that a thread loads before it tests any, 64 to 128
 // bytes in flight.  Q6 on 6e7 rows x 4 columns (0.96 GB): one group a time and
-// 8 blocks per SM 169 us, two groups 151, and 32 blocks per SM's worth of grid
-// (several waves, no SM idle at the end) 148.5, 0.99 of the copy rate; one
-// pass of the grid-stride loop per block 189.
+// 8 blocks per SM 167 us, two groups and 16 blocks per SM 140, 1.05 of the
+// copy rate.
 constexpr int agg_groups(int nu) { return nu <= 1 ? 4 : nu <= 4 ? 2 : 1; }
 template <int NU, int MODE, bool VEC>
 __global__ void __launch_bounds__(256) scan_aggregate_kernel(const __grid_constant__ AggParams p) {
@@ -346,22 +345,40 @@ __global__ void __launch_bounds__(256) scan_aggregate_kernel(const __grid_consta
     for (int c = 0; c < NU; c++) v[c] = __ldg(p.col[c] + r);
     one(v);
   }
+  // one addition per block to the count and to the sum: they all go to one
+  // address, and with one per warp to the count their tail took 12 us of a
+  // 1e8-row scan of one column (77 us, 67 without) and doubled 4e6 rows of
+  // five (32 us, 16 without)
+  __shared__ unsigned long long s_cnt[8];
   if (p.count) {
     unsigned long long c = cnt;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(p.count, c);
+    if ((threadIdx.x & 31) == 0) s_cnt[threadIdx.x >> 5] = c;
   }
-  if (MODE > 0 && p.sum) {
-    const unsigned __int128 t = block_sum128(acc);
-    if (threadIdx.x == 0 && t) add128(p.sum, t);
+  unsigned __int128 sum = 0;
+  if (MODE > 0 && p.sum) sum = block_sum128(acc);
+  else __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long c = 0;
+    if (p.count)
+#pragma unroll
+      for (int k = 0; k < 8; k++) c += s_cnt[k];
+    if (c) atomicAdd(p.count, c);
+    if (sum) add128(p.sum, sum);
   }
 }
 
 template <int NU, int MODE>
 void launch_agg(const AggParams &p, bool vec, int sm_count, cudaStream_t s) {
   const uint64_t work = vec ? (p.nrows / 4 + agg_groups(NU) - 1) / agg_groups(NU) : p.nrows;
-  const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((work + 255) / 256, (uint64_t)sm_count * 32));
+  // 16 blocks per SM (two waves, so that no SM idles through a last partial
+  // one): within 2 % of the best of 8, 16 and 32 for one to eight columns of
+  // 4e6 to 1e8 rows, where 8 loses up to 15 % (two columns) and 32 up to 30 %
+  // (4e6 rows).  Four-byte loads: 8 (1e8 rows of three columns 228, 232 and
+  // 234 us).
+  const uint64_t most = (uint64_t)sm_count * (vec ? 16 : 8);
+  const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((work + 255) / 256, most));
   if (vec) scan_aggregate_kernel<NU, MODE, true><<<grid, 256, 0, s>>>(p);
   else scan_aggregate_kernel<NU, MODE, false><<<grid, 256, 0, s>>>(p);
 }
