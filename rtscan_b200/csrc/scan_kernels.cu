@@ -29,7 +29,6 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
-constexpr uint64_t kClusterMaxValues = 1u << 19;  // see launch_scan_small
 
 __device__ __forceinline__ uint4 ld_stream(const uint32_t *p) {
   uint4 v;
@@ -170,6 +169,8 @@ __global__ void __launch_bounds__(kThreads) scan_fused_kernel(const __grid_const
 // first.
 constexpr int kClusterThreads = 512;
 constexpr int kClusterCtas = 8;
+constexpr uint64_t kClusterTiles = kClusterCtas * (kClusterThreads / 32);  // see launch_scan_small
+constexpr uint64_t kClusterMaxValues = 1u << 19;
 template <int NT, bool VEC>
 __global__ void __launch_bounds__(kClusterThreads) scan_cluster_kernel(const __grid_constant__ ScanParams p) {
   __shared__ uint32_t part[kClusterThreads / 32];
@@ -331,11 +332,14 @@ void launch_scan_fused(const ScanParams &p, bool vector_ok, cudaStream_t s) {
 }
 
 bool launch_scan_small(const ScanParams &p, bool vector_ok, cudaStream_t s) {
-  // One launch instead of a memset and a launch: 1e5 rows 12.2 -> 10.3 us a
-  // call among others (the host's enqueue), 15.4 against 18.3 us apart.  Eight
-  // SMs keep up with the whole chip to about here: at 5e5 values 15.4 us
-  // against 17.6 for memset and scan.
-  if (p.nrows * (uint64_t)p.nterms > kClusterMaxValues) return false;
+  // One launch instead of a memset and a launch: 1e5 rows 12.7 -> 10.8 us a
+  // call among others (the host's enqueue), 21.2 against 20.1 us apart.  As
+  // long as each of the cluster's warps has one tile (and 2^19 values in all):
+  // past that its eight SMs take a second round, which columns that are not
+  // 16-byte aligned feel at once (1.6e5 rows of two: 33 us, memset and scan
+  // 19) and aligned ones from 4e5 rows (12.8 and 12.1 us).
+  const uint64_t ntiles = (p.nrows + kTileRows - 1) / kTileRows;
+  if (ntiles > kClusterTiles || p.nrows * (uint64_t)p.nterms > kClusterMaxValues) return false;
   cudaError_t e;
   if (vector_ok) {
     switch (p.nterms) {
