@@ -142,7 +142,7 @@ void fused(rts_ctx *ctx, const Plan &plan, uint32_t *out, unsigned long long *co
     p.full_tiles = n / rts::kTileRows;
     if (!one || !rts::launch_scan_small(p, vec, s)) {
       if (one) RTS_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), s));
-      rts::launch_scan_fused(p, vec, s);
+      rts::launch_scan_fused(p, vec, ctx->sm_count, s);
     }
     launches++;
   }
@@ -428,7 +428,7 @@ rts_status rts_scan_separate_async(rts_ctx *ctx, const rts_term *terms, int32_t 
       p.out = i == 0 ? dev_bitmap : scratch_bitmap(ctx, 0);
       p.nrows = n;
       p.full_tiles = n / rts::kTileRows;
-      rts::launch_scan_fused(p, aligned16(p.t[0].col), s);
+      rts::launch_scan_fused(p, aligned16(p.t[0].col), ctx->sm_count, s);
       launches++;
       if (i > 0) {
         rts::launch_bitmap_op(RTS_BM_AND, dev_bitmap, dev_bitmap, p.out, words, 0, ctx->sm_count, s);

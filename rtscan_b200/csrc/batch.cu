@@ -911,7 +911,7 @@ int launch_outside(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std::
       sp.nrows = n;
       sp.full_tiles = n / kTileRows;
       if (first == 0) RTS_CUDA(cudaMemsetAsync(counts + o, 0, 8, s));
-      launch_scan_fused(sp, vec, s);
+      launch_scan_fused(sp, vec, ctx->sm_count, s);
       launches++;
     }
   }
@@ -1514,7 +1514,7 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
         sp.count = counts + f.slot_query[j];
         sp.nrows = row_end - row_begin;
         sp.full_tiles = sp.nrows / kTileRows;
-        launch_scan_fused(sp, vec, s);
+        launch_scan_fused(sp, vec, ctx->sm_count, s);
         launches++;
       }
       continue;

@@ -135,7 +135,7 @@ rts_status scan_separate_noalloc(const uint32_t *const *dev_cols, int32_t ncols,
       p.out = i == 0 ? dev_bitmap : d.scratch;
       p.nrows = nrows;
       p.full_tiles = nrows / rts::kTileRows;
-      rts::launch_scan_fused(p, aligned16(p.t[0].col), s);
+      rts::launch_scan_fused(p, aligned16(p.t[0].col), d.sm_count, s);
       if (i > 0) rts::launch_bitmap_op(RTS_BM_AND, dev_bitmap, dev_bitmap, d.scratch, words, 0, d.sm_count, s);
     }
     e = cudaMemsetAsync(count, 0, 8, s);

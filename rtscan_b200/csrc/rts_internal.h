@@ -129,7 +129,7 @@ struct LaunchShape {
   int blocks;
   int threads;
 };
-void launch_scan_fused(const ScanParams &p, bool vector_ok, cudaStream_t s);  // adds to *p.count
+void launch_scan_fused(const ScanParams &p, bool vector_ok, int sm_count, cudaStream_t s);  // adds to *p.count
 // A small table's scan whose count is stored, not added (nothing zeroes it
 // before); false, with nothing launched, when the table is not small.
 bool launch_scan_small(const ScanParams &p, bool vector_ok, cudaStream_t s);

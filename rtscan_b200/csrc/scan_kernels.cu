@@ -29,6 +29,7 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kThreads = 256;
+constexpr int kScalarCtas = 8;  // per SM, of a scan of unaligned columns
 
 __device__ __forceinline__ uint4 ld_stream(const uint32_t *p) {
   uint4 v;
@@ -156,7 +157,6 @@ __device__ __forceinline__ uint32_t scan_tiles(const ScanParams &p, uint64_t war
   return cnt;
 }
 
-// One tile per warp (see launch_nt).
 template <int NT, bool VEC>
 __global__ void __launch_bounds__(kThreads) scan_fused_kernel(const __grid_constant__ ScanParams p) {
   const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -203,12 +203,14 @@ __global__ void __launch_bounds__(kClusterThreads) scan_cluster_kernel(const __g
 // One tile per warp: the hardware hands CTAs to SMs as they finish, so no SM
 // idles through a last partial round (3 columns of 3e7 rows: 6.2 rounds of
 // persistent warps took 73.7 us, one tile per warp 63.5; 1e8 rows 188 and
-// 178 us, one column of 1e8 rows 65.5 and 63.5 us).
+// 178 us, one column of 1e8 rows 65.5 and 63.5 us).  Columns that are not
+// 16-byte aligned: as many CTAs as are resident, in rounds (one column of 1e8
+// rows 214 us, one tile per warp 234; two of 3e7 rows 143 and 150).
 template <int NT, bool VEC>
-void launch_nt(const ScanParams &p, cudaStream_t s) {
+void launch_nt(const ScanParams &p, int sm_count, cudaStream_t s) {
   const uint64_t ntiles = (p.nrows + kTileRows - 1) / kTileRows;
   const uint64_t want = (ntiles + (kThreads / 32) - 1) / (kThreads / 32);
-  const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, 0x7FFFFFFFull));
+  const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, VEC ? 0x7FFFFFFFull : (uint64_t)sm_count * kScalarCtas));
   scan_fused_kernel<NT, VEC><<<blocks, kThreads, 0, s>>>(p);
 }
 
@@ -317,17 +319,17 @@ int grid_for(uint64_t items, int per_thread, int sm_count) {
 
 }  // namespace
 
-void launch_scan_fused(const ScanParams &p, bool vector_ok, cudaStream_t s) {
+void launch_scan_fused(const ScanParams &p, bool vector_ok, int sm_count, cudaStream_t s) {
   if (vector_ok) {
     switch (p.nterms) {
-      case 1: launch_nt<1, true>(p, s); break;
-      case 2: launch_nt<2, true>(p, s); break;
-      case 3: launch_nt<3, true>(p, s); break;
-      case 4: launch_nt<4, true>(p, s); break;
-      default: launch_nt<0, true>(p, s); break;
+      case 1: launch_nt<1, true>(p, sm_count, s); break;
+      case 2: launch_nt<2, true>(p, sm_count, s); break;
+      case 3: launch_nt<3, true>(p, sm_count, s); break;
+      case 4: launch_nt<4, true>(p, sm_count, s); break;
+      default: launch_nt<0, true>(p, sm_count, s); break;
     }
   } else {
-    launch_nt<0, false>(p, s);
+    launch_nt<0, false>(p, sm_count, s);
   }
 }
 
