@@ -857,6 +857,7 @@ struct BatchPlan {
     int groups;   // 32-slot groups of the pass (table words per position)
     bool few;     // at most kFewMaxQueries queries: batch_few_kernel, no tables in the blob
     FewPass fp;
+    FewParams fk;  // its parameters (results and range are set at the launch)
     int pre_slot = -1;  // shared positions: this pass's slot in the scratch, or -1
     // a further group of passes sharing positions, and the slot in it (both
     // -1: the pass searches)
@@ -1231,6 +1232,7 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
     BatchPlan::Pass b;
     memset(&b.bp, 0, sizeof b.bp);
     memset(&b.fp, 0, sizeof b.fp);
+    memset(&b.fk, 0, sizeof b.fk);
     b.few = false;
     const int C = (int)pp.cols.size();
     if (variant == 4 && (int)pp.qs.size() <= kFewMaxQueries) {
@@ -1256,11 +1258,21 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
         }
       }
       std::vector<uint32_t> B;
+      uint32_t at = 0;
+      b.fk.nq = fp.nq;
+      b.fk.vec = 1;
       for (int c = 0; c < C; c++) {
-        B = std::move(pp.bounds[c].vals);
-        std::sort(B.begin(), B.end());
-        std::copy(B.begin(), B.end(), fp.bnd[c]);
-        pre_shape(B, fp.shape[c], few_buckets(C, ctx->nrows));
+        if (fp.nq <= few_direct_max(C)) {
+          for (int j = 0; j < few_direct_max(C); j++) memcpy(b.fk.tab + 2 * (j * C + c), &fp.term[j][c], 8);
+        } else {
+          B = std::move(pp.bounds[c].vals);
+          std::sort(B.begin(), B.end());
+          PreCol shape;
+          pre_shape(B, shape, few_buckets(C, ctx->nrows));
+          at = few_column(b.fk, fp, c, B, shape, at);
+        }
+        b.fk.col[c] = fp.col[c];
+        b.fk.vec = b.fk.vec && ((uintptr_t)fp.col[c] & 15) == 0;
       }
       b.off = plan.blob.size();
       plan.passes.push_back(b);
@@ -1520,25 +1532,22 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
       continue;
     }
     if (b.few) {
-      FewPass fp = b.fp;
+      FewParams fp = b.fk;
+      memcpy(fp.slot_query, b.fp.slot_query, sizeof fp.slot_query);  // (without the dropped queries)
       fp.out = out;
       fp.stride_words = stride_words;
       fp.counts = counts;
       fp.nrows = row_end;
       fp.words = words_for(ctx->nrows);
-      fp.tile_begin = row_begin / 1024;
-      fp.ntiles = (row_end + 1023) / 1024;
-      fp.vec = 1;
-      for (int c = 0; c < fp.ncols; c++) fp.vec = fp.vec && ((uintptr_t)fp.col[c] & 15) == 0;
-      switch (fp.ncols) {
-        case 1: launch_few<1>(fp, ctx->sm_count, s); break;
-        case 2: launch_few<2>(fp, ctx->sm_count, s); break;
-        case 3: launch_few<3>(fp, ctx->sm_count, s); break;
-        case 4: launch_few<4>(fp, ctx->sm_count, s); break;
-        case 5: launch_few<5>(fp, ctx->sm_count, s); break;
-        case 6: launch_few<6>(fp, ctx->sm_count, s); break;
-        case 7: launch_few<7>(fp, ctx->sm_count, s); break;
-        default: launch_few<8>(fp, ctx->sm_count, s); break;
+      switch (b.fp.ncols) {
+        case 1: launch_few<1>(fp, row_begin, ctx->sm_count, s); break;
+        case 2: launch_few<2>(fp, row_begin, ctx->sm_count, s); break;
+        case 3: launch_few<3>(fp, row_begin, ctx->sm_count, s); break;
+        case 4: launch_few<4>(fp, row_begin, ctx->sm_count, s); break;
+        case 5: launch_few<5>(fp, row_begin, ctx->sm_count, s); break;
+        case 6: launch_few<6>(fp, row_begin, ctx->sm_count, s); break;
+        case 7: launch_few<7>(fp, row_begin, ctx->sm_count, s); break;
+        default: launch_few<8>(fp, row_begin, ctx->sm_count, s); break;
       }
       launches++;
       continue;
