@@ -7,10 +7,10 @@
 // kernels are HBM-bound streaming passes:
 //
 //   * rts_bitmap_rows_async: ordered compaction of a bitmap into ascending
-//     uint32 row ids.  Pass 1 counts the set bits of each 1024-word tile;
-//     pass 2 reloads each tile, sums the counts before it (past 2^28 rows a
-//     one-CTA scan does) and every warp expands its words one at a time, a
-//     lane per bit.  Bytes: 2 x N/8 read + 4 per row id.
+//     uint32 row ids.  Pass 1 counts the set bits of each block's tiles of
+//     1024 words (one tile, four on large tables); pass 2 reloads them, sums
+//     the counts before its block (past 2^30 rows a one-CTA scan does) and
+//     expands the words.  Bytes: 2 x N/8 read + 4 per row id.
 //   * rts_bitmap_sum_async: sum of a column, or of the product of two
 //     columns, over the set rows (128-bit exact).  A warp takes 1024 rows:
 //     its 32 bitmap words, then the values as 16-byte loads, each lane
@@ -36,17 +36,19 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kCompactThreads = 256;
 constexpr int kCompactRounds = 4;                                   // words per thread
 constexpr int kCompactTileWords = kCompactThreads * kCompactRounds;  // 1024 words = 32768 rows
+constexpr int kCompactGroup = 4;  // tiles of a block on large tables
 constexpr int kScanThreads = 1024;
-// Up to this many tiles (2^28 rows) every block of the write pass sums the
-// counts of the tiles before it itself (at most 32 loads per thread, from
-// L2); a scan launch of one block costs about 3 us.
-constexpr uint64_t kCompactSelfTiles = 8192;
+// Up to this many blocks (2^30 rows) every block of the write pass sums the
+// counts of the blocks before it itself (at most 32 loads per thread, from
+// L2); a scan launch of one block costs 3 us and more.
+constexpr uint64_t kCompactSelfBlocks = 8192;
+constexpr uint32_t kCompactDense = 3000;  // ids of a warp's 128 words, see compact_write_kernel
 
 // The thread's kCompactRounds words of the tile: warp w's round r holds words
 // 32 * (kCompactRounds * w + r) .. + 31 of it, one per lane.
 __device__ __forceinline__ void compact_words(const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask,
-                                              uint32_t (&x)[kCompactRounds]) {
-  const uint64_t w0 = (uint64_t)blockIdx.x * kCompactTileWords + (threadIdx.x >> 5) * (32 * kCompactRounds) +
+                                              uint64_t tile, uint32_t (&x)[kCompactRounds]) {
+  const uint64_t w0 = tile * kCompactTileWords + (threadIdx.x >> 5) * (32 * kCompactRounds) +
                       (threadIdx.x & 31);
 #pragma unroll
   for (int r = 0; r < kCompactRounds; r++) {
@@ -55,34 +57,41 @@ __device__ __forceinline__ void compact_words(const uint32_t *__restrict__ bm, u
   }
 }
 
+// Set bits of every block's tiles.
+template <int TILES>
 __global__ void __launch_bounds__(kCompactThreads) compact_count_kernel(const uint32_t *__restrict__ bm,
                                                                         uint64_t words, uint32_t tail_mask,
-                                                                        uint32_t *__restrict__ tile_count) {
-  uint32_t x[kCompactRounds];
-  compact_words(bm, words, tail_mask, x);
+                                                                        uint32_t *__restrict__ block_count) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t c = 0;
 #pragma unroll
-  for (int r = 0; r < kCompactRounds; r++) c += __popc(x[r]);
+  for (int t = 0; t < TILES; t++) {
+    uint32_t x[kCompactRounds];
+    compact_words(bm, words, tail_mask, (uint64_t)blockIdx.x * TILES + t, x);
+#pragma unroll
+    for (int r = 0; r < kCompactRounds; r++) c += __popc(x[r]);
+  }
   c = __reduce_add_sync(kFull, c);
   __shared__ uint32_t part[kCompactThreads / 32];
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
+  if (lane == 0) part[warp] = c;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t v = threadIdx.x < kCompactThreads / 32 ? part[threadIdx.x] : 0u;
-    v = __reduce_add_sync(kFull, v);
-    if (threadIdx.x == 0) tile_count[blockIdx.x] = v;
+  if (threadIdx.x == 0) {
+    uint32_t v = 0;
+#pragma unroll
+    for (int k = 0; k < kCompactThreads / 32; k++) v += part[k];
+    block_count[blockIdx.x] = v;
   }
 }
 
-// One CTA: exclusive prefix of the tile counts (as uint64) and the total.
-__global__ void __launch_bounds__(kScanThreads) compact_scan_kernel(const uint32_t *__restrict__ tile_count,
-                                                                    uint64_t ntiles,
-                                                                    unsigned long long *__restrict__ tile_off,
+// One CTA: exclusive prefix of the block counts (as uint64) and the total.
+__global__ void __launch_bounds__(kScanThreads) compact_scan_kernel(const uint32_t *__restrict__ block_count,
+                                                                    uint64_t nblocks,
+                                                                    unsigned long long *__restrict__ block_off,
                                                                     unsigned long long *__restrict__ total) {
-  const uint64_t per = (ntiles + kScanThreads - 1) / kScanThreads;
-  const uint64_t b = threadIdx.x * per, e = std::min<uint64_t>(ntiles, b + per);
+  const uint64_t per = (nblocks + kScanThreads - 1) / kScanThreads;
+  const uint64_t b = threadIdx.x * per, e = std::min<uint64_t>(nblocks, b + per);
   unsigned long long s = 0;
-  for (uint64_t i = b; i < e; i++) s += tile_count[i];
+  for (uint64_t i = b; i < e; i++) s += block_count[i];
   // block-wide inclusive scan of the thread sums
   __shared__ unsigned long long warp_sum[kScanThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -106,100 +115,133 @@ __global__ void __launch_bounds__(kScanThreads) compact_scan_kernel(const uint32
   __syncthreads();
   unsigned long long off = warp_sum[warp] + incl - s;
   for (uint64_t i = b; i < e; i++) {
-    tile_off[i] = off;
-    off += tile_count[i];
+    block_off[i] = off;
+    off += block_count[i];
   }
   if (threadIdx.x == kScanThreads - 1) *total = off;
 }
 
-// A warp expands its words one at a time: lane l holds bit l's row, so a
-// word's ids leave as one run of consecutive addresses (the pass before had
-// every thread store the ids of 16 words at its own place: 32 lines per
-// store instruction).  tile_off null: the block sums the counts before its
-// tile, and the last block stores the total.
-// Bound by issue, about 12 instructions per nonzero word (and one POPC), then
-// by the id writes.  2^25 rows, a two-column scan of 10-50 % and its row ids:
-// 127 -> 82 us a pass; of that the write pass takes 29 us and the count 3.
+// A lane takes one word at a time, its ids go to the warp's buffer at the
+// word's place, and the warp copies the buffer out as one run of consecutive
+// addresses; where nearly every bit is set (kCompactDense) the warp takes a
+// word at a time instead, a lane per bit.  (Every thread storing its ids of 16
+// words straight to memory: 32 lines per store instruction; a lane per bit
+// everywhere: 12 instructions per nonzero word, however few bits it has.)
+// block_off null: the block sums the counts before its tiles, and the last
+// block stores the total.
+// Bound by issue, seven instructions per bit of a round's fullest word and
+// five per 32 ids copied, then by the id writes.  Row ids of a bitmap, both
+// passes (us; straight stores, a lane per bit, this): 2^25 rows at 3 % 23, 25,
+// 15, at 50 % 107, 33, 27; 1e8 rows at 1 % 23, 37, 25, at 10 % 72, 80, 37, at
+// 100 % 1221, 81, 82; 6e8 rows at 1 % 82, 183, 97, at 50 % 2979, 445, 356.
+template <int TILES>
 __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
-    const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask, const uint32_t *__restrict__ tile_count,
-    const unsigned long long *__restrict__ tile_off, uint32_t *__restrict__ rows, uint64_t capacity,
+    const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask, const uint32_t *__restrict__ block_count,
+    const unsigned long long *__restrict__ block_off, uint32_t *__restrict__ rows, uint64_t capacity,
     unsigned long long *__restrict__ total) {
-  __shared__ unsigned long long s_before[kCompactThreads / 32];
-  __shared__ uint32_t s_warp[kCompactThreads / 32];
+  constexpr int kWarps = kCompactThreads / 32;
+  __shared__ unsigned long long s_before[kWarps];
+  __shared__ uint32_t s_warp[2][kWarps];
+  __shared__ __align__(16) uint32_t s_ids[kWarps][33 * 32];  // a round's ids in order, the i-th at i + i / 32
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x[kCompactRounds];
-  compact_words(bm, words, tail_mask, x);
+  const bool last = blockIdx.x == gridDim.x - 1;
+  const uint32_t tile0 = blockIdx.x * TILES;
+  uint32_t next[kCompactRounds];
+  compact_words(bm, words, tail_mask, tile0, next);
+  if (TILES > 1 && !last && __ldg(block_count + blockIdx.x) == 0) return;  // (the last block may store the total)
   unsigned long long before = 0;
-  if (!tile_off) {
-    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kCompactThreads) before += __ldg(tile_count + i);
+  if (!block_off)
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kCompactThreads) before += __ldg(block_count + i);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(kFull, before, o);
-    if (lane == 0) s_before[warp] = before;
-  }
-  // inclusive scans of the rounds' popcounts over the lanes, two rounds to a
-  // word (a round has at most 1024 bits)
-  static_assert(kCompactRounds == 4, "two packed scans");
-  uint32_t c01 = __popc(x[0]) | __popc(x[1]) << 16, c23 = __popc(x[2]) | __popc(x[3]) << 16;
-  const uint32_t own01 = c01, own23 = c23;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(kFull, before, o);
+  if (lane == 0) s_before[warp] = before;
+  unsigned long long base = block_off ? block_off[blockIdx.x] : 0ull;
+  uint32_t *const ids = s_ids[warp];
+#pragma unroll 1
+  for (int t = 0; t < TILES; t++) {
+    uint32_t x[kCompactRounds];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y01 = __shfl_up_sync(kFull, c01, o), y23 = __shfl_up_sync(kFull, c23, o);
-    if (lane >= o) {
-      c01 += y01;
-      c23 += y23;
+    for (int r = 0; r < kCompactRounds; r++) x[r] = next[r];
+    if (t + 1 < TILES) compact_words(bm, words, tail_mask, tile0 + t + 1, next);
+    // exclusive scans of the rounds' popcounts over the lanes, two rounds to a
+    // word (a round has at most 1024 bits)
+    static_assert(kCompactRounds == 4, "two packed scans");
+    uint32_t c01 = __popc(x[0]) | __popc(x[1]) << 16, c23 = __popc(x[2]) | __popc(x[3]) << 16;
+    const uint32_t own01 = c01, own23 = c23;
+    if (__any_sync(kFull, (c01 | c23) != 0)) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y01 = __shfl_up_sync(kFull, c01, o), y23 = __shfl_up_sync(kFull, c23, o);
+        if (lane >= o) {
+          c01 += y01;
+          c23 += y23;
+        }
+      }
     }
-  }
-  const uint32_t all01 = __shfl_sync(kFull, c01, 31), all23 = __shfl_sync(kFull, c23, 31);
-  c01 -= own01;
-  c23 -= own23;
-  const uint32_t sum[kCompactRounds] = {all01 & 0xFFFFu, all01 >> 16, all23 & 0xFFFFu, all23 >> 16};
-  if (lane == 0) s_warp[warp] = sum[0] + sum[1] + sum[2] + sum[3];
-  __syncthreads();
-  uint32_t start = 0, tile = 0;  // ids of the tile before this warp, in the tile
+    const uint32_t all01 = __shfl_sync(kFull, c01, 31), all23 = __shfl_sync(kFull, c23, 31);
+    c01 -= own01;
+    c23 -= own23;
+    const uint32_t sum[kCompactRounds] = {all01 & 0xFFFFu, all01 >> 16, all23 & 0xFFFFu, all23 >> 16};
+    if (lane == 0) s_warp[t & 1][warp] = sum[0] + sum[1] + sum[2] + sum[3];
+    __syncthreads();  // (the other buffer's readers are a barrier behind)
+    if (t == 0) {
 #pragma unroll
-  for (int k = 0; k < kCompactThreads / 32; k++) {
-    if (k < warp) start += s_warp[k];
-    tile += s_warp[k];
-  }
-  unsigned long long base = 0;
-  if (tile_off) {
-    base = tile_off[blockIdx.x];
-  } else {
+      for (int k = 0; k < kWarps; k++) base += s_before[k];
+    }
+    uint32_t start = 0, tile = 0;  // ids of the tile before this warp, in the tile
 #pragma unroll
-    for (int k = 0; k < kCompactThreads / 32; k++) base += s_before[k];
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = base + tile;
-  }
-  if (base >= capacity) return;
-  // the warp's nonzero words, each with its index and its ids' offset in the tile
-  __shared__ uint2 s_word[kCompactThreads / 32][32 * kCompactRounds];
-  uint2 *const list = s_word[warp];
-  int n = 0;
+    for (int k = 0; k < kWarps; k++) {
+      if (k < warp) start += s_warp[t & 1][k];
+      tile += s_warp[t & 1][k];
+    }
+    if (base < capacity && (all01 | all23) != 0) {
+      uint32_t *const dst = rows + base;
+      const uint32_t room = (uint32_t)std::min<unsigned long long>(capacity - base, tile);
+      const uint32_t row0 = (uint32_t)(((uint64_t)(tile0 + t) * kCompactTileWords + warp * (32 * kCompactRounds)) * 32);
+      const uint32_t all = sum[0] + sum[1] + sum[2] + sum[3];
+      if (all > kCompactDense && start + all <= room) {
+        // the warp's nonzero words, each with its index and its ids' offset in
+        // the tile; then a word at a time, a lane per bit
+        uint2 *const list = reinterpret_cast<uint2 *>(ids);
+        int n = 0;
 #pragma unroll
-  for (int r = 0; r < kCompactRounds; r++) {
-    const uint32_t off = start + (r == 0 ? c01 & 0xFFFFu : r == 1 ? c01 >> 16 : r == 2 ? c23 & 0xFFFFu : c23 >> 16);
-    const unsigned some = __ballot_sync(kFull, x[r] != 0);
-    if (x[r]) list[n + __popc(some & ((1u << lane) - 1))] = make_uint2(x[r], off | (uint32_t)(32 * r + lane) << 16);
-    n += __popc(some);
-    start += sum[r];
-  }
-  __syncwarp();
-  uint32_t *const dst = rows + base;
-  const uint32_t row = (uint32_t)(((uint64_t)blockIdx.x * kCompactTileWords + warp * (32 * kCompactRounds)) * 32) + lane;
-  const uint32_t bit = 0x80000000u >> lane, above = ~(0xFFFFFFFFu >> lane);  // MSB-first: bit 31 is the word's first row
-  const uint32_t room = (uint32_t)std::min<unsigned long long>(capacity - base, 0xFFFFFFFFull);
-  if (room >= tile) {
+        for (int r = 0; r < kCompactRounds; r++) {
+          const uint32_t at =
+              start + (r == 0 ? c01 & 0xFFFFu : r == 1 ? c01 >> 16 : r == 2 ? c23 & 0xFFFFu : c23 >> 16);
+          const unsigned some = __ballot_sync(kFull, x[r] != 0);
+          if (x[r]) list[n + __popc(some & ((1u << lane) - 1))] = make_uint2(x[r], at | (uint32_t)(32 * r + lane) << 16);
+          n += __popc(some);
+          start += sum[r];
+        }
+        __syncwarp();
+        const uint32_t bit = 0x80000000u >> lane, above = ~(0xFFFFFFFFu >> lane);
 #pragma unroll 4
-    for (int k = 0; k < n; k++) {
-      const uint2 w = list[k];
-      if (w.x & bit) dst[(w.y & 0xFFFFu) + __popc(w.x & above)] = row + ((w.y >> 16) << 5);
+        for (int k = 0; k < n; k++) {
+          const uint2 w = list[k];
+          if (w.x & bit) dst[(w.y & 0xFFFFu) + __popc(w.x & above)] = row0 + lane + ((w.y >> 16) << 5);
+        }
+        __syncwarp();
+      } else {
+#pragma unroll
+        for (int r = 0; r < kCompactRounds; r++) {
+          uint32_t at = r == 0 ? c01 & 0xFFFFu : r == 1 ? c01 >> 16 : r == 2 ? c23 & 0xFFFFu : c23 >> 16;
+          const uint32_t row = row0 + 32 * (32 * r + lane);
+          for (uint32_t w = x[r]; w; at++) {  // MSB-first: bit 31 is the word's first row
+            const int b = __clz(w);
+            ids[at + (at >> 5)] = row + b;
+            w &= 0x7FFFFFFFu >> b;
+          }
+          __syncwarp();
+          for (uint32_t i = lane; i < sum[r]; i += 32)
+            if (start + i < room) dst[start + i] = ids[i + (i >> 5)];
+          __syncwarp();
+          start += sum[r];
+        }
+      }
     }
-  } else {
-    for (int k = 0; k < n; k++) {
-      const uint2 w = list[k];
-      const uint32_t at = (w.y & 0xFFFFu) + __popc(w.x & above);
-      if ((w.x & bit) && at < room) dst[at] = row + ((w.y >> 16) << 5);
-    }
+    base += tile;
   }
+  if (!block_off && last && threadIdx.x == 0) *total = base;
 }
 
 // 128-bit accumulation: per-thread unsigned __int128, one pair of 64-bit
@@ -397,7 +439,7 @@ void launch_agg_nu(int nu, const AggParams &p, bool vec, int sm_count, cudaStrea
   }
 }
 
-// Device scratch for the compaction's tile counts and offsets (grown as needed).
+// Device scratch for the compaction's block counts and offsets (grown as needed).
 void *agg_scratch(rts_ctx *ctx, size_t bytes) {
   if (ctx->agg_bytes < bytes) {
     if (ctx->agg_dev) cudaFree(ctx->agg_dev);
@@ -439,16 +481,21 @@ rts_status rts_bitmap_rows_async(rts_ctx *ctx, const uint32_t *dev_bitmap, uint6
     }
     const uint32_t tail_mask = (nrows & 31) ? ~(0xFFFFFFFFu >> (nrows & 31)) : 0xFFFFFFFFu;
     const uint64_t ntiles = (words + rts::kCompactTileWords - 1) / rts::kCompactTileWords;
-    const bool self = ntiles <= rts::kCompactSelfTiles;
-    char *scratch = static_cast<char *>(rts::agg_scratch(ctx, ntiles * 12 + 16));
-    auto *tile_off = self ? nullptr : reinterpret_cast<unsigned long long *>(scratch);
-    auto *tile_count = reinterpret_cast<uint32_t *>(scratch + ntiles * 8);
+    // four tiles per block once every SM has eight such blocks: 2.5e8 rows at
+    // 1 % 47 us, a tile per block 52, but 1e8 rows at 50 % 88 and 70
+    const bool group = ntiles >= (uint64_t)ctx->sm_count * 8 * rts::kCompactGroup;
+    const uint64_t nblocks = group ? (ntiles + rts::kCompactGroup - 1) / rts::kCompactGroup : ntiles;
+    const bool self = nblocks <= rts::kCompactSelfBlocks;
+    char *scratch = static_cast<char *>(rts::agg_scratch(ctx, nblocks * 12 + 16));
+    auto *block_off = self ? nullptr : reinterpret_cast<unsigned long long *>(scratch);
+    auto *block_count = reinterpret_cast<uint32_t *>(scratch + nblocks * 8);
     auto *total = reinterpret_cast<unsigned long long *>(dev_count);
-    rts::compact_count_kernel<<<(unsigned)ntiles, rts::kCompactThreads, 0, s>>>(dev_bitmap, words, tail_mask,
-                                                                               tile_count);
-    if (!self) rts::compact_scan_kernel<<<1, rts::kScanThreads, 0, s>>>(tile_count, ntiles, tile_off, total);
-    rts::compact_write_kernel<<<(unsigned)ntiles, rts::kCompactThreads, 0, s>>>(
-        dev_bitmap, words, tail_mask, tile_count, tile_off, dev_rows, capacity, total);
+    const auto count = group ? rts::compact_count_kernel<rts::kCompactGroup> : rts::compact_count_kernel<1>;
+    const auto write = group ? rts::compact_write_kernel<rts::kCompactGroup> : rts::compact_write_kernel<1>;
+    count<<<(unsigned)nblocks, rts::kCompactThreads, 0, s>>>(dev_bitmap, words, tail_mask, block_count);
+    if (!self) rts::compact_scan_kernel<<<1, rts::kScanThreads, 0, s>>>(block_count, nblocks, block_off, total);
+    write<<<(unsigned)nblocks, rts::kCompactThreads, 0, s>>>(dev_bitmap, words, tail_mask, block_count, block_off,
+                                                             dev_rows, capacity, total);
     RTS_CUDA(cudaGetLastError());
     ctx->launches += self ? 2 : 3;
     return RTS_OK;
