@@ -439,21 +439,51 @@ void launch_agg_nu(int nu, const AggParams &p, bool vec, int sm_count, cudaStrea
   }
 }
 
-// Device scratch for the compaction's block counts and offsets (grown as needed).
-void *agg_scratch(rts_ctx *ctx, size_t bytes) {
-  if (ctx->agg_bytes < bytes) {
-    if (ctx->agg_dev) cudaFree(ctx->agg_dev);
-    ctx->agg_dev = nullptr;
-    ctx->agg_bytes = 0;
-    if (cudaMalloc(&ctx->agg_dev, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      throw Error(RTS_ERR_NOMEM, "aggregate scratch allocation failed");
+// Device scratch for a compaction's block counts and offsets on stream s.  The
+// context's calls share one buffer (grown as needed), each ordered after the
+// one before, whatever their streams (agg_done).  A captured call runs when its
+// graph is launched, so it gets a buffer of its own, which stays until the
+// context goes.
+struct AggScratch {
+  rts_ctx *ctx;
+  cudaStream_t s;
+  void *dev = nullptr;
+  bool captured = false;
+  AggScratch(rts_ctx *c, size_t bytes, cudaStream_t stream) : ctx(c), s(stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();
+    captured = st != cudaStreamCaptureStatusNone;
+    if (captured) {
+      ctx->agg_captured.reserve(ctx->agg_captured.size() + 1);
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (an allocation is no part of the capture)
+      RTS_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      const bool ok = cudaMalloc(&dev, bytes) == cudaSuccess;
+      RTS_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      if (!ok) fail_alloc();
+      ctx->agg_captured.push_back(dev);
+      return;
     }
-    ctx->agg_bytes = bytes;
+    if (!ctx->agg_done) RTS_CUDA(cudaEventCreateWithFlags(&ctx->agg_done, cudaEventDisableTiming));
+    if (ctx->agg_bytes < bytes) {
+      RTS_CUDA(cudaEventSynchronize(ctx->agg_done));
+      if (ctx->agg_dev) cudaFree(ctx->agg_dev);
+      ctx->agg_dev = nullptr;
+      ctx->agg_bytes = 0;
+      if (cudaMalloc(&ctx->agg_dev, bytes) != cudaSuccess) fail_alloc();
+      ctx->agg_bytes = bytes;
+    }
+    dev = ctx->agg_dev;
+    RTS_CUDA(cudaStreamWaitEvent(s, ctx->agg_done, 0));
   }
-  return ctx->agg_dev;
-}
-
+  // The call's last use of the buffer has been queued.
+  void done() {
+    if (!captured) RTS_CUDA(cudaEventRecord(ctx->agg_done, s));
+  }
+  static void fail_alloc() {
+    cudaGetLastError();
+    throw Error(RTS_ERR_NOMEM, "aggregate scratch allocation failed");
+  }
+};
 
 rts_status fail(rts_ctx *ctx, const std::exception &e) {
   if (ctx) ctx->err = e.what();
@@ -486,7 +516,8 @@ rts_status rts_bitmap_rows_async(rts_ctx *ctx, const uint32_t *dev_bitmap, uint6
     const bool group = ntiles >= (uint64_t)ctx->sm_count * 8 * rts::kCompactGroup;
     const uint64_t nblocks = group ? (ntiles + rts::kCompactGroup - 1) / rts::kCompactGroup : ntiles;
     const bool self = nblocks <= rts::kCompactSelfBlocks;
-    char *scratch = static_cast<char *>(rts::agg_scratch(ctx, nblocks * 12 + 16));
+    rts::AggScratch buffer(ctx, nblocks * 12 + 16, s);
+    char *scratch = static_cast<char *>(buffer.dev);
     auto *block_off = self ? nullptr : reinterpret_cast<unsigned long long *>(scratch);
     auto *block_count = reinterpret_cast<uint32_t *>(scratch + nblocks * 8);
     auto *total = reinterpret_cast<unsigned long long *>(dev_count);
@@ -496,7 +527,9 @@ rts_status rts_bitmap_rows_async(rts_ctx *ctx, const uint32_t *dev_bitmap, uint6
     if (!self) rts::compact_scan_kernel<<<1, rts::kScanThreads, 0, s>>>(block_count, nblocks, block_off, total);
     write<<<(unsigned)nblocks, rts::kCompactThreads, 0, s>>>(dev_bitmap, words, tail_mask, block_count, block_off,
                                                              dev_rows, capacity, total);
-    RTS_CUDA(cudaGetLastError());
+    const cudaError_t launched = cudaGetLastError();
+    buffer.done();
+    RTS_CUDA(launched);
     ctx->launches += self ? 2 : 3;
     return RTS_OK;
   } catch (const std::exception &e) {

@@ -191,6 +191,8 @@ rts_ctx::~rts_ctx() {
   if (small_dev) cudaFree(small_dev);
   if (query_slots) cudaFree(query_slots);
   if (agg_dev) cudaFree(agg_dev);
+  if (agg_done) cudaEventDestroy(agg_done);
+  for (void *p : agg_captured) cudaFree(p);
   if (batch) rts::destroy_batch(batch);
   if (host_batch) rts::destroy_host_batch(host_batch);
 }

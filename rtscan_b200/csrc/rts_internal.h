@@ -245,8 +245,10 @@ struct rts_ctx {
   void *small_dev = nullptr;
   rts::QuerySlot *query_slots = nullptr;  // BinDex query launches (rts::kQuerySlots, used in turn)
   uint64_t query_next = 0;
-  void *agg_dev = nullptr;    // compaction scratch (tile counts and offsets)
+  void *agg_dev = nullptr;    // compaction scratch (block counts and offsets)
   size_t agg_bytes = 0;
+  cudaEvent_t agg_done = nullptr;    // after its last use
+  std::vector<void *> agg_captured;  // buffers of captured compactions
   rts::BatchScratch *batch = nullptr;
   rts::HostBatchBuffers *host_batch = nullptr;
   rts::BatchConfig batch_cfg;
