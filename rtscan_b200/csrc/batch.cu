@@ -747,8 +747,21 @@ struct BoundSet {
     vals.push_back(v);
   }
   size_t size() const { return vals.size(); }
+  // Sort vals; rank(v) of a member v is then its place among them.
+  void close() {
+    std::sort(vals.begin(), vals.end());
+    ranks.resize(cell.size());
+    for (uint32_t k = 0; k < vals.size(); k++) ranks[at(vals[k])] = k;
+  }
+  uint32_t rank(uint32_t v) const { return ranks[at(v)]; }
 
  private:
+  std::vector<uint32_t> ranks;  // of every cell's value
+  uint32_t at(uint32_t v) const {
+    uint32_t i = home(v);
+    while (cell[i] != v) i = (i + 1) & (uint32_t)(cell.size() - 1);
+    return i;
+  }
   void put(uint32_t v) {
     uint32_t i = home(v);
     while (cell[i] != 0) i = (i + 1) & (uint32_t)(cell.size() - 1);
@@ -765,8 +778,7 @@ struct PassPlan {
 // Shared-memory bytes of a pass's tables, boundaries and bucket index for
 // the given boundary counts (bucket index at most 4097 uint16 per column).
 size_t column_bytes(size_t m, int G) {
-  size_t nb = 1;
-  while (nb < 4 * m && nb < 4096) nb <<= 1;
+  const size_t nb = m == 0 ? 1 : m >= 1024 ? 4096 : (size_t)1 << (32 - __builtin_clz((uint32_t)(4 * m - 1)));
   return (m + 1) * (size_t)G * 4 + m * 4 + (nb + 2) * 2 + 8;
 }
 
@@ -948,11 +960,11 @@ std::vector<uint16_t> bucket_index(const std::vector<uint32_t> &B, uint64_t span
   };
   // the index of a bucket map over nb buckets: first boundary whose bucket is >= k
   auto index = [&](uint32_t nb, auto &&bucket) {
-    std::vector<uint16_t> bk(nb + 1);
-    uint32_t i = 0;
-    for (uint32_t k = 0; k <= nb; k++) {
-      while (i < m && bucket(B[i] - bmin) < k) i++;
-      bk[k] = (uint16_t)i;
+    std::vector<uint16_t> bk(nb + 1, (uint16_t)m);
+    uint32_t k = 0;
+    for (uint32_t i = 0; i < m; i++) {
+      const uint32_t at = bucket(B[i] - bmin);  // the buckets from k up to it start at i
+      for (; k <= at; k++) bk[k] = (uint16_t)i;
     }
     return bk;
   };
@@ -982,9 +994,9 @@ int pass_groups(int nq) { return nq <= 128 ? 4 : nq <= 256 ? 8 : 16; }
 // Bucket shape of a column's sorted distinct boundaries B (pc.m, origin, M,
 // L, nbk) with at most max_buckets buckets, the last one past every
 // boundary (values above them all need no search).  Candidates: linear
-// buckets, and for M = 1..12 the log-linear ones with the smallest L that
-// fits; the one with the fewest search steps per row wins, fewer buckets on
-// a tie.  Query bounds sit at value quantiles, so every interval between
+// buckets, and log-linear ones of M = 2, 5, 8 and 11 with the smallest L that
+// fits, then the best M's neighbours; the one with the fewest search steps
+// per row wins, fewer buckets on a tie.  Query bounds sit at value quantiles, so every interval between
 // neighbouring boundaries stands for the same share of the rows, spread
 // evenly over its values: a bucket with boundaries inside costs their search
 // steps times the shares of the intervals that it overlaps.
@@ -1039,26 +1051,35 @@ void pre_shape(const std::vector<uint32_t> &B, PreCol &pc, uint32_t max_buckets)
     t.origin = B[0] > (1u << L) ? B[0] - (1u << L) : 0;
     t.nbk = 0xFFFFFFFFu;
     const uint32_t last = M == 31 ? (B.back() - t.origin) >> L : pre_bucket(t, B.back());
-    t.nbk = last >= max_buckets ? 0 : last + 2;
+    t.nbk = last + 2 > max_buckets ? 0 : last + 2;
     return t;
   };
-  PreCol best;
-  for (uint32_t L = 0;; L++) {
-    best = shape(31, L);
-    if (best.nbk && best.nbk <= max_buckets) break;
+  // the smallest L that fits, of linear buckets (at 0) and of every M; more
+  // buckets per octave need no smaller one
+  PreCol fit[13];
+  for (uint32_t i = 0, L = 0; i <= 12; i++) {
+    if (i < 2) L = 0;
+    while (L < 32 && !(fit[i] = shape(i ? i : 31, L)).nbk) L++;
   }
-  double best_cost = cost_of(best, 1e300);
-  for (uint32_t M = 1; M <= 12; M++)
-    for (uint32_t L = 0; L < 32; L++) {
-      const PreCol t = shape(M, L);
-      if (!t.nbk || t.nbk > max_buckets) continue;
-      const double cost = cost_of(t, best_cost);
-      if (cost < best_cost || (cost == best_cost && t.nbk < best.nbk)) {
-        best_cost = cost;
-        best = t;
-      }
-      break;
+  PreCol best;
+  double best_cost = 1e300;
+  int best_i = -1;
+  auto consider = [&](int i) {
+    const PreCol &t = fit[i];
+    if (!t.nbk) return;
+    const double cost = cost_of(t, best_cost);
+    if (cost < best_cost || (cost == best_cost && t.nbk < best.nbk)) {
+      best_cost = cost;
+      best = t;
+      best_i = i;
     }
+  };
+  for (const int i : {8, 0, 5, 11, 2}) consider(i);
+  const int near = best_i;
+  if (near > 0) {  // the next values of M
+    consider(near - 1);
+    if (near < 12) consider(near + 1);
+  }
   pc = best;
 }
 
@@ -1068,15 +1089,19 @@ std::vector<uint32_t> pre_buckets(const std::vector<uint32_t> &B, PreCol &pc,
   pre_shape(B, pc, max_buckets);
   if (B.empty()) return {0u};
   const uint32_t m = pc.m;
-  // the index: entry k = base | n << 16 (see PreCol)
-  std::vector<uint32_t> ent(pc.nbk);
-  uint32_t lo = 0;
-  for (uint32_t k = 0; k < pc.nbk; k++) {
-    uint32_t hi = lo;
-    while (hi < m && (k + 1 == pc.nbk || pre_bucket(pc, B[hi]) == k)) hi++;
-    const uint64_t start = (uint64_t)pc.origin + pre_bucket_start(pc.M, pc.L, k);
-    const uint32_t base = lo + (lo < hi && B[lo] == start ? 1u : 0u);
-    ent[k] = base | (hi - base) << 16;
+  // the index: entry k = base | n << 16 (see PreCol); between the buckets that
+  // hold boundaries it stays the same
+  std::vector<uint32_t> ent(pc.nbk, m);
+  uint32_t k = 0;
+  for (uint32_t lo = 0; lo < m;) {
+    const uint32_t at = pre_bucket(pc, B[lo]);
+    uint32_t hi = lo + 1;
+    while (hi < m && pre_bucket(pc, B[hi]) == at) hi++;
+    std::fill(ent.begin() + k, ent.begin() + at, lo);
+    const uint64_t start = (uint64_t)pc.origin + pre_bucket_start(pc.M, pc.L, at);
+    const uint32_t base = lo + (B[lo] == start ? 1u : 0u);
+    ent[at] = base | (hi - base) << 16;
+    k = at + 1;
     lo = hi;
   }
   return ent;
@@ -1286,8 +1311,8 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
     std::vector<uint32_t> blob;
     std::vector<std::vector<uint32_t>> B(C);
     for (int c = 0; c < C; c++) {
+      pp.bounds[c].close();
       B[c] = std::move(pp.bounds[c].vals);
-      std::sort(B[c].begin(), B[c].end());
       bp.m[c] = (uint32_t)B[c].size();
     }
     // tables: row pos holds, per slot, whether the values of interval pos
@@ -1310,13 +1335,10 @@ BatchPlan build_plan(rts_ctx *ctx, const std::vector<NormQuery> &norm, const std
       const NormQuery &q = norm[pp.qs[i]];
       for (size_t k = 0; k < q.cols.size(); k++) {
         const int c = (int)(std::find(pp.cols.begin(), pp.cols.end(), q.cols[k]) - pp.cols.begin());
-        const std::vector<uint32_t> &Bc = B[c];
+        const BoundSet &Bc = pp.bounds[c];
         const uint32_t m = bp.m[c];
-        const uint32_t p0 =
-            q.lo[k] > 0 ? (uint32_t)(std::lower_bound(Bc.begin(), Bc.end(), q.lo[k]) - Bc.begin()) + 1 : 0u;
-        const uint32_t p1 = q.hi[k] < 0xFFFFFFFFu
-                                ? (uint32_t)(std::lower_bound(Bc.begin(), Bc.end(), q.hi[k] + 1) - Bc.begin())
-                                : m;
+        const uint32_t p0 = q.lo[k] > 0 ? Bc.rank(q.lo[k]) + 1 : 0u;
+        const uint32_t p1 = q.hi[k] < 0xFFFFFFFFu ? Bc.rank(q.hi[k] + 1) : m;
         uint32_t *tab = blob.data() + bp.tab_off[c];
         tab[(size_t)p0 * Gp + grp] ^= bit;
         if (p1 + 1 <= m) tab[(size_t)(p1 + 1) * Gp + grp] ^= bit;
