@@ -882,7 +882,7 @@ struct BatchPlan {
   std::vector<Pass> passes;
   std::vector<uint32_t> blob;
   // shared positions of the passes with a pre_slot (npass 0: none)
-  PreParams pre;
+  PreParams pre = {};
   size_t pre_off = 0;  // word offset of the union boundaries, buckets and maps in `blob`
   std::vector<Group> groups;
   // batch_plan_drop: per query index, where its slot is (built at the first
