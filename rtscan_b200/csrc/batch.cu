@@ -1061,7 +1061,7 @@ void pre_shape(const std::vector<uint32_t> &B, PreCol &pc, uint32_t max_buckets)
     if (i < 2) L = 0;
     while (L < 32 && !(fit[i] = shape(i ? i : 31, L)).nbk) L++;
   }
-  PreCol best;
+  PreCol best = {};
   double best_cost = 1e300;
   int best_i = -1;
   auto consider = [&](int i) {
