@@ -116,6 +116,7 @@ struct rts_server {
   std::atomic<int64_t> waiting{0};    // requests in the inbox and the queue
   std::atomic<bool> idle{false};      // the worker is about to wait on cv_work
   std::atomic<bool> failed{false};    // `fatal` is set
+  std::atomic<uint64_t> freed{0};     // slots that fetches and cancels gave back
   int cursor = 0;
   uint64_t active_version = 1, plan_version = 0;
   uint64_t plan_step = 0;                // steps launched when the running plan was made
@@ -243,6 +244,35 @@ struct rts_server {
       lk.lock();
     }
     if (!news) wait_work(lk, std::chrono::microseconds(200));
+  }
+
+  // With the result pool full and requests queued, slots come back one fetch
+  // at a time, and a step per slot keeps `mu` from the next fetch: wait until an
+  // eighth of the pool is free, or no slot came back for kGatherPause, or
+  // kGatherMost has passed (mu held through lk on both sides).  500 requests on
+  // a pool of 256 and 1.7e7 rows x 2 columns: 7.5 -> 3.7 ms, 2e5 rows x 4
+  // columns 8.0 -> 3.9.
+  static constexpr double kGatherPause = 20e-6, kGatherMost = 100e-6;
+  void gather_slots(std::unique_lock<std::mutex> &lk) {
+    const size_t enough = std::max<size_t>(1, slots.size() / 8);
+    auto few = [&] { return !queue.empty() && !free_slots.empty() && free_slots.size() < std::min(queue.size(), enough); };
+    drain_inbox();
+    if (!few()) return;
+    const double t0 = now_s();
+    double last = t0, t = t0;
+    uint64_t was = freed.load();
+    while (few() && t - last < kGatherPause && t - t0 < kGatherMost && !stop.load()) {
+      lk.unlock();
+      do {
+        std::this_thread::yield();
+        t = now_s();
+      } while (freed.load() == was && t - last < kGatherPause);
+      lk.lock();
+      if (freed.load() != was) {
+        was = freed.load();
+        last = t;
+      }
+    }
   }
 
   // Admit queued requests into free slots (mu held); their counts are
@@ -447,6 +477,7 @@ struct rts_server {
         {
           std::unique_lock<std::mutex> lk(mu);
           for (auto e : retired) put_event(e);
+          gather_slots(lk);
           admit();
           fence_cancels();
           reap();
@@ -721,6 +752,7 @@ rts_status rts_server_fetch(rts_server *srv, uint64_t ticket, uint32_t *host_bit
         S.state = FREE;
         srv->ticket_slot.erase(it);
         srv->free_slots.push_back(sl);
+        srv->freed++;
         srv->cv_work.notify_one();
         return RTS_OK;
       }
@@ -740,6 +772,7 @@ rts_status rts_server_fetch(rts_server *srv, uint64_t ticket, uint32_t *host_bit
     S.state = FREE;
     srv->ticket_slot.erase(ticket);
     srv->free_slots.push_back(sl);
+    srv->freed++;
     srv->cv_work.notify_one();
     return RTS_OK;
   });
@@ -772,6 +805,7 @@ rts_status rts_server_cancel(rts_server *srv, uint64_t ticket) {
     } else if (S.state == DONE) {
       S.state = FREE;
       srv->free_slots.push_back(it->second);
+      srv->freed++;
     }
     srv->ticket_slot.erase(it);
     srv->cancelled++;
