@@ -1975,7 +1975,21 @@ extern "C" rts_status rts_scan_batch_host(rts_ctx *ctx, const uint32_t *const *h
     }
     // Finish chunk r once its counts are on the host: the dense queries'
     // words leave as one 2D copy per run of consecutive dense queries, the
-    // packed ones as masks and values expanded by the pool.
+    // packed ones as masks and values expanded by the pool.  A copy costs about
+    // 2 us beside its bytes: where dense queries lie between packed ones and
+    // the chunks are short, their words wait for up to kHoldChunks chunks and
+    // leave together (1000 queries on 1.6e7 rows, every second one packed: 8
+    // chunks 43.5 ms, 3 chunks 36.7, this 32.6).
+    constexpr int kHoldChunks = 4, kHoldRuns = 32;
+    const bool short_chunks = chunk_rows < (1u << 22);
+    constexpr uint64_t kNothing = ~0ull;
+    std::vector<uint64_t> held(nq, kNothing);  // first word of a query's words that wait
+    auto download = [&](int q, int n, uint64_t from, uint64_t to) {
+      RTS_CUDA(cudaMemcpy2DAsync(host_bitmaps + (uint64_t)q * stride_words + from, stride_words * 4,
+                                 H.bitmaps + (uint64_t)q * stride_words + from, stride_words * 4, (to - from) * 4,
+                                 (size_t)n, cudaMemcpyDeviceToHost, H.copy));
+      H.last_d2h += (to - from) * 4 * (uint64_t)n;
+    };
     auto finish = [&](int r) {
       const uint64_t r0 = (uint64_t)r * chunk_rows, r1 = std::min<uint64_t>(nrows, r0 + chunk_rows);
       const uint64_t w0 = r0 / 32, w1 = r1 == nrows ? words : r1 / 32, cw = w1 - w0;
@@ -1993,27 +2007,31 @@ extern "C" rts_status rts_scan_batch_host(rts_ctx *ctx, const uint32_t *const *h
         return try_pack && packed_words(i) * rts::kPackDen <= cw * rts::kPackNum &&
                total + packed_words(i) <= max_packed;
       };
-      int q = 0;
-      while (q < nq) {
-        if (is_outside[q]) {
-          q++;
-          continue;
-        }
-        if (packs(q)) {
-          const uint64_t c = packed_words(q);
+      int runs = 0;
+      bool in_run = false;
+      for (int q = 0; q < nq; q++) {
+        const bool pack = !is_outside[q] && packs(q), dense = !is_outside[q] && !pack;
+        if (pack) {
+          if (held[q] != kNothing) download(q, 1, held[q], w0);
+          held[q] = kNothing;
           qlh[packed.size()] = q;
           qoh[packed.size()] = total;
           packed.push_back(q);
-          total += c;
-          q++;
-          continue;
+          total += packed_words(q);
+        } else if (dense && held[q] == kNothing) {
+          held[q] = w0;
         }
-        int qb = q + 1;  // a run of dense queries
-        while (qb < nq && !is_outside[qb] && !packs(qb)) qb++;
-        RTS_CUDA(cudaMemcpy2DAsync(host_bitmaps + (uint64_t)q * stride_words + w0, stride_words * 4,
-                                   H.bitmaps + (uint64_t)q * stride_words + w0, stride_words * 4, cw * 4,
-                                   (size_t)(qb - q), cudaMemcpyDeviceToHost, H.copy));
-        H.last_d2h += cw * 4 * (uint64_t)(qb - q);
+        runs += dense && !in_run;
+        in_run = dense;
+      }
+      const bool hold = short_chunks && runs > kHoldRuns && r % kHoldChunks != kHoldChunks - 1 && r != nchunks - 1;
+      for (int q = 0; q < nq && !hold;) {
+        int qb = q + 1;
+        if (held[q] != kNothing) {  // a run of dense queries
+          while (qb < nq && held[qb] == held[q]) qb++;
+          download(q, qb - q, held[q], w1);
+          std::fill(held.begin() + q, held.begin() + qb, kNothing);
+        }
         q = qb;
       }
       if (packed.empty()) return;
