@@ -1480,11 +1480,13 @@ void launch_pre(rts_ctx *ctx, PreParams P, cudaStream_t s) {
 
 // Launch every pass of `plan` (blob already on the device) over rows
 // [row_begin, row_end); row_begin is a multiple of 4096 (the largest block
-// of the pass shapes).  Returns launches.
+// of the pass shapes).  Returns launches; *searched (may be null) tells whether
+// a pass searched its own positions.
 int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_t *out, uint64_t stride_words,
                 unsigned long long *counts, uint64_t row_begin, uint64_t row_end, void *scratch,
-                size_t scratch_bytes, cudaStream_t s) {
+                size_t scratch_bytes, cudaStream_t s, bool *searched = nullptr) {
   int launches = 0;
+  if (searched) *searched = false;
   // the passes of each group that shares positions, when the caller's scratch
   // holds them: the positions, then the passes (the scratch is the next
   // group's after that); the others search their own
@@ -1587,6 +1589,7 @@ int launch_plan(rts_ctx *ctx, BatchPlan &plan, const uint32_t *dev_blob, uint32_
     bp.nblocks = (row_end + rows_per_block - 1) / rows_per_block;
     bp.vec_store = (((uintptr_t)out & 15) == 0 && stride_words % 4 == 0) ? 1 : 0;
     bp.word_bytes = 4;
+    if (searched) *searched = true;
     const bool w8 = ctx->batch_cfg.warps_per_cta == 8;
     if (b.variant == 4) {
       if (b.cmax == 4) {
@@ -1690,7 +1693,9 @@ void context_pre_done(rts_ctx *ctx, cudaStream_t s) {
 }
 
 void batch_scan(rts_ctx *ctx, const rts_term *terms, const int32_t *offsets, int nq, uint32_t *out,
-                uint64_t stride_words, unsigned long long *counts, cudaStream_t s, size_t table_budget) {
+                uint64_t stride_words, unsigned long long *counts, cudaStream_t s, size_t table_budget,
+                bool *searched) {
+  if (searched) *searched = false;
   std::vector<NormQuery> norm = normalize_all(ctx, terms, offsets, nq);
   std::vector<int> inside, outside;
   for (int q = 0; q < nq; q++) (runs_in_kernel(norm[q]) ? inside : outside).push_back(q);
@@ -1703,7 +1708,8 @@ void batch_scan(rts_ctx *ctx, const rts_term *terms, const int32_t *offsets, int
     const uint32_t *dev_blob = upload_plan(ctx, plan, s, &done);
     const size_t pre_bytes = plan_pre_bytes(plan, ctx->nrows);
     void *pre = context_pre_scratch(ctx, pre_bytes, s);
-    launches += launch_plan(ctx, plan, dev_blob, out, stride_words, counts, 0, ctx->nrows, pre, pre_bytes, s);
+    launches +=
+        launch_plan(ctx, plan, dev_blob, out, stride_words, counts, 0, ctx->nrows, pre, pre_bytes, s, searched);
     if (pre) context_pre_done(ctx, s);
     RTS_CUDA(cudaEventRecord(done, s));
   }

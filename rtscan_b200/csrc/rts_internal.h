@@ -210,18 +210,20 @@ struct BatchScratch;
 void destroy_batch(BatchScratch *b);
 struct HostBatchBuffers;
 void destroy_host_batch(HostBatchBuffers *b);
-// Launch shape of the batched kernels: the variant, warps per CTA (variant
-// 3: 8 or 16), queries per pass (<= 512 for variant 4, <= 256 for 3) and the
+// Launch shape of the batched kernels: the variant, warps per CTA (8 or 16; of
+// the passes that search their own positions), queries per pass (<= 512 for variant 4, <= 256 for 3) and the
 // shared-memory bytes a pass may spend on its mask tables (the rest of the
 // CTA's shared memory stages result words and row positions).
 struct BatchConfig {
   int variant = 4;                // 4: passes of up to 512 queries over CTA-wide blocks; 3: 256-query passes per warp
-  int warps_per_cta = 16;         // variant 3 only
+  int warps_per_cta = 16;         // variant 3, and variant 4's passes that search their own positions
   int max_queries_per_pass = 512;
   size_t table_budget = 136 * 1024;
 };
+// *searched (may be null): whether a table pass searched its own positions.
 void batch_scan(rts_ctx *ctx, const rts_term *terms, const int32_t *offsets, int nq, uint32_t *out,
-                uint64_t stride_words, unsigned long long *counts, cudaStream_t s, size_t table_budget);
+                uint64_t stride_words, unsigned long long *counts, cudaStream_t s, size_t table_budget,
+                bool *searched = nullptr);
 
 }  // namespace rts
 

@@ -1,22 +1,23 @@
 // Autotuner for the batched kernel's launch shape.
 //
-// The batched kernel's speed depends on three knobs that trade shared memory
-// against each other: warps per CTA (each warp stages 8 KB of result words),
-// queries per pass (more queries share each row's interval lookups but need
-// larger mask tables) and the mask-table budget (which fixes how many
-// queries fit a pass and how many CTAs fit an SM).  rts_autotune_batch runs
-// every candidate on a row sample of the resident table with the caller's
-// queries, keeps the fastest, and can cache the choice in a small text file
-// keyed by GPU, SM count, column count, table size and batch size.
+// The batched kernel's speed depends on three knobs: queries per pass (more
+// queries share each row's positions but need larger mask tables), the
+// mask-table budget (which fixes how many queries fit a pass and how many CTAs
+// fit an SM), and, for passes that search their own positions, warps per CTA.
+// rts_autotune_batch runs every candidate on a row sample of the resident table
+// with the caller's queries, keeps the fastest, and can cache the choice in a
+// small text file keyed by GPU, SM count, column count, table size and batch
+// size.
 //
-// Candidates: variant 4 (pass shapes of 128/256/512 slots) with 16-warp
-// CTAs at seven pass sizes from 128 to 512 queries and two table budgets,
-// and with 8-warp CTAs (one per SM, or two when small tables leave room),
-// and variant 3 at 8 and 16 warps per CTA with two budgets each.  The sample
-// is the table's first rows: as many as the result bitmaps of the batch fit
-// in a quarter of the free device memory, at least 2^24 and at most 2^27
-// (all of a smaller table).  Each candidate runs once untimed and twice
-// timed; the report (rts_autotune_report) lists every candidate's time.
+// Candidates: variant 4 (pass shapes of 128/256/512 slots) at seven pass sizes
+// from 128 to 512 queries and two table budgets, three more with a small
+// budget, and two that differ from earlier ones in warps per CTA only, which
+// run only where a pass searches its own positions (the others would time the
+// same launches twice); and variant 3 at 8 and 16 warps per CTA with two budgets
+// each.  The sample is the table's first rows: as many as the result bitmaps of
+// the batch fit in a quarter of the free device memory, at least 2^24 and at
+// most 2^27 (all of a smaller table).  Each candidate runs once untimed and
+// twice timed; the report (rts_autotune_report) lists every candidate's time.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -39,13 +40,20 @@ std::vector<Candidate> candidates() {
   std::vector<Candidate> c;
   for (int qpp : {512, 448, 384, 320, 256, 192, 128})
     for (size_t budget : {(size_t)136 * 1024, (size_t)112 * 1024}) c.push_back({4, 16, qpp, budget});
-  // 8-warp CTAs: one per SM with large tables, or two per SM when the
-  // tables stay under about 56 KiB
+  // 8-warp CTAs, for passes that search their own positions: one per SM with
+  // large tables (see twin), or two per SM when the tables stay under about 56
+  // KiB
   for (int qpp : {512, 256}) c.push_back({4, 8, qpp, (size_t)136 * 1024});
   for (int qpp : {512, 256, 128}) c.push_back({4, 8, qpp, (size_t)56 * 1024});
   for (size_t budget : {(size_t)88 * 1024, (size_t)64 * 1024}) c.push_back({3, 16, 256, budget});
   for (size_t budget : {(size_t)140 * 1024, (size_t)40 * 1024}) c.push_back({3, 8, 256, budget});
   return c;
+}
+
+// Whether b differs from a in warps per CTA only, which passes that read shared
+// positions do not depend on.
+bool twin(const Candidate &a, const Candidate &b) {
+  return a.variant == 4 && b.variant == 4 && a.qpp == b.qpp && a.budget == b.budget;
 }
 
 size_t max_budget(int variant, int warps) {
@@ -178,12 +186,16 @@ rts_status rts_autotune_batch(rts_ctx *ctx, const rts_term *terms, const int32_t
     const rts::BatchConfig dflt;
     double default_ms = -1;
     bool first = true;
+    std::vector<Candidate> shared;  // timed, with no pass searching its own positions
     for (const Candidate &c : candidates()) {
+      if (std::any_of(shared.begin(), shared.end(), [&](const Candidate &d) { return twin(c, d); })) continue;
       ctx->batch_cfg.variant = c.variant;
       ctx->batch_cfg.warps_per_cta = c.warps;
       ctx->batch_cfg.max_queries_per_pass = c.qpp;
       ctx->batch_cfg.table_budget = c.budget;
-      rts::batch_scan(ctx, terms, offsets, nq, bm, stride, cnt, nullptr, c.budget);  // warm-up
+      bool searched = false;
+      rts::batch_scan(ctx, terms, offsets, nq, bm, stride, cnt, nullptr, c.budget, &searched);  // warm-up
+      if (!searched) shared.push_back(c);
       RTS_CUDA(cudaEventRecord(e0, nullptr));
       for (int r = 0; r < 2; r++) rts::batch_scan(ctx, terms, offsets, nq, bm, stride, cnt, nullptr, c.budget);
       RTS_CUDA(cudaEventRecord(e1, nullptr));
