@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(kScanThreads) compact_scan_kernel(const uint32
 // Bound by issue, seven instructions per bit of a round's fullest word and
 // five per 32 ids copied, then by the id writes.  Row ids of a bitmap, both
 // passes (us; straight stores, a lane per bit, this): 2^25 rows at 3 % 23, 25,
-// 15, at 50 % 107, 33, 27; 1e8 rows at 1 % 23, 37, 25, at 10 % 72, 80, 37, at
-// 100 % 1221, 81, 82; 6e8 rows at 1 % 82, 183, 97, at 50 % 2979, 445, 356.
+// 13, at 50 % 107, 33, 27; 1e8 rows at 1 % 23, 37, 23, at 10 % 74, 80, 31, at
+// 100 % 1253, 81, 82; 6e8 rows at 1 % 82, 184, 85, at 50 % 3078, 446, 358.
 template <int TILES>
 __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
     const uint32_t *__restrict__ bm, uint64_t words, uint32_t tail_mask, const uint32_t *__restrict__ block_count,
@@ -222,20 +222,26 @@ __global__ void __launch_bounds__(kCompactThreads) compact_write_kernel(
         }
         __syncwarp();
       } else {
+        // through the buffer: all the rounds' ids at once where they fit it
+        const bool together = all <= 32 * 32;
+        uint32_t off = 0;
 #pragma unroll
         for (int r = 0; r < kCompactRounds; r++) {
-          uint32_t at = r == 0 ? c01 & 0xFFFFu : r == 1 ? c01 >> 16 : r == 2 ? c23 & 0xFFFFu : c23 >> 16;
+          uint32_t at = off + (r == 0 ? c01 & 0xFFFFu : r == 1 ? c01 >> 16 : r == 2 ? c23 & 0xFFFFu : c23 >> 16);
           const uint32_t row = row0 + 32 * (32 * r + lane);
           for (uint32_t w = x[r]; w; at++) {  // MSB-first: bit 31 is the word's first row
             const int b = __clz(w);
             ids[at + (at >> 5)] = row + b;
             w &= 0x7FFFFFFFu >> b;
           }
+          off += sum[r];
+          if (together && r + 1 < kCompactRounds) continue;
           __syncwarp();
-          for (uint32_t i = lane; i < sum[r]; i += 32)
+          for (uint32_t i = lane; i < off; i += 32)
             if (start + i < room) dst[start + i] = ids[i + (i >> 5)];
           __syncwarp();
-          start += sum[r];
+          start += off;
+          off = 0;
         }
       }
     }
@@ -512,7 +518,7 @@ rts_status rts_bitmap_rows_async(rts_ctx *ctx, const uint32_t *dev_bitmap, uint6
     const uint32_t tail_mask = (nrows & 31) ? ~(0xFFFFFFFFu >> (nrows & 31)) : 0xFFFFFFFFu;
     const uint64_t ntiles = (words + rts::kCompactTileWords - 1) / rts::kCompactTileWords;
     // four tiles per block once every SM has eight such blocks: 2.5e8 rows at
-    // 1 % 47 us, a tile per block 52, but 1e8 rows at 50 % 88 and 70
+    // 1 % 39 us, a tile per block 52, but 1e8 rows at 50 % 88 and 66
     const bool group = ntiles >= (uint64_t)ctx->sm_count * 8 * rts::kCompactGroup;
     const uint64_t nblocks = group ? (ntiles + rts::kCompactGroup - 1) / rts::kCompactGroup : ntiles;
     const bool self = nblocks <= rts::kCompactSelfBlocks;
