@@ -547,7 +547,7 @@ GpuBinDex::~GpuBinDex() {
   if (base) cudaFree(base);
 }
 
-uint32_t *GpuBinDex::allocate(uint64_t rows, int areas, std::unique_ptr<GpuBinDex> old) {
+uint32_t *GpuBinDex::allocate(uint64_t rows, int areas, std::unique_ptr<GpuBinDex> old, size_t extra) {
   n = rows;
   K = areas;
   fv_stride = (((n + 31) >> 5) + 3) / 4 * 4;
@@ -558,7 +558,7 @@ uint32_t *GpuBinDex::allocate(uint64_t rows, int areas, std::unique_ptr<GpuBinDe
     return (words + to - 1) / to * to;
   };
   const uint64_t col_words = padded(n), fv_words = padded((uint64_t)(K - 1) * fv_stride);
-  const size_t bytes = (2 * col_words + fv_words + padded(bindex_table_words(n, K))) * 4;
+  const size_t bytes = (2 * col_words + fv_words + padded(bindex_table_words(n, K))) * 4 + extra;
   if (old && old->cap >= bytes && old->cap <= 2 * bytes) {
     RTS_CUDA(cudaDeviceSynchronize());  // queries that still read the old index, on any stream
     std::swap(base, old->base);
@@ -613,16 +613,25 @@ std::unique_ptr<GpuBinDex> build_bindex(const uint32_t *col, uint64_t n, int K, 
   if (n < (uint64_t)K) throw Error(RTS_ERR_ARG, "BinDex needs at least K rows");
   if (n >= (1ull << 32)) throw Error(RTS_ERR_ARG, "BinDex supports fewer than 2^32 rows per column");
   auto b = std::make_unique<GpuBinDex>();
-  uint32_t *tables = b->allocate(n, K, std::move(old));
   // row ids and sort scratch: in the filter vectors' place, which are written
-  // after the sort, when they fit (K >= 98 or so), else for the call
+  // after the sort, when they fit (K >= 98 or so); else with the index when
+  // small (a device allocation costs 0.3 ms, as does giving it back: 1e5 rows
+  // and K = 16 took 1.09 ms, 0.5 so), else for the call
   size_t temp_bytes = 0;
-  RTS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, col, b->sval, b->spos, b->spos, (int64_t)n, 0, 32, s));
-  const uint64_t ids_words = (n + 63) / 64 * 64, fv_words = (uint64_t)(K - 1) * b->fv_stride;
+  uint32_t *const none = nullptr;
+  RTS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, col, none, none, none, (int64_t)n, 0, 32, s));
+  const uint64_t ids_words = (n + 63) / 64 * 64;
+  const size_t scratch = ids_words * 4 + (temp_bytes + 255) / 256 * 256;
+  const bool in_fv = scratch <= (uint64_t)(K - 1) * ((((n + 31) >> 5) + 3) / 4 * 4) * 4;
+  constexpr size_t kKept = 2 << 20;
+  const size_t kept = !in_fv && scratch <= kKept ? scratch : 0;
+  uint32_t *tables = b->allocate(n, K, std::move(old), kept);
   DevFree f_temp{nullptr};
   uint32_t *ids = b->fv;
-  if (ids_words * 4 + temp_bytes > fv_words * 4) {
-    ids = dev_alloc<uint32_t>(ids_words + (temp_bytes + 3) / 4);
+  if (kept) {
+    ids = tables + (bindex_table_words(n, K) + 63) / 64 * 64;
+  } else if (!in_fv) {
+    ids = dev_alloc<uint32_t>(scratch / 4);
     f_temp.p = ids;
   }
   void *temp = ids + ids_words;

@@ -166,8 +166,9 @@ struct GpuBinDex {
   // Room for an index of n rows and K areas (fields n, K, fv_stride, sval,
   // spos, fv are set), in `old`'s allocation when that is large enough and at
   // most twice as large (one device allocation costs 0.4-2 ms here), else a
-  // new one; returns the tables (bindex_table_words() words, 8-byte aligned).
-  uint32_t *allocate(uint64_t n, int K, std::unique_ptr<GpuBinDex> old);
+  // new one, with `extra` bytes behind the tables; returns the tables
+  // (bindex_table_words() words, 256-byte aligned).
+  uint32_t *allocate(uint64_t n, int K, std::unique_ptr<GpuBinDex> old, size_t extra = 0);
   ~GpuBinDex();
 };
 constexpr int kSampleStride = 1024;
