@@ -192,6 +192,7 @@ rts_ctx::~rts_ctx() {
   if (query_slots) cudaFree(query_slots);
   if (agg_dev) cudaFree(agg_dev);
   if (agg_done) cudaEventDestroy(agg_done);
+  if (scratch_done) cudaEventDestroy(scratch_done);
   for (void *p : agg_captured) cudaFree(p);
   if (batch) rts::destroy_batch(batch);
   if (host_batch) rts::destroy_host_batch(host_batch);
@@ -422,6 +423,16 @@ rts_status rts_scan_separate_async(rts_ctx *ctx, const rts_term *terms, int32_t 
     }
     const uint64_t n = ctx->nrows, words = rts::words_for(n);
     int launches = 0;
+    // The terms after the first go through a bitmap of the context: this call's
+    // use of it comes after the last call's, whatever their streams.  (Not
+    // under capture, where that would be a dependency on work outside the graph.)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
+    const bool ordered = plan.terms.size() > 1 && capture == cudaStreamCaptureStatusNone;
+    if (ordered) {
+      if (!ctx->scratch_done) RTS_CUDA(cudaEventCreateWithFlags(&ctx->scratch_done, cudaEventDisableTiming));
+      RTS_CUDA(cudaStreamWaitEvent(s, ctx->scratch_done, 0));
+    }
     for (size_t i = 0; i < plan.terms.size(); i++) {
       rts::ScanParams p;
       memset(&p, 0, sizeof p);
@@ -437,6 +448,7 @@ rts_status rts_scan_separate_async(rts_ctx *ctx, const rts_term *terms, int32_t 
         launches++;
       }
     }
+    if (ordered) RTS_CUDA(cudaEventRecord(ctx->scratch_done, s));
     if (dev_count) {
       RTS_CUDA(cudaMemsetAsync(dev_count, 0, 8, s));
       rts::launch_bitmap_count(dev_bitmap, n, reinterpret_cast<unsigned long long *>(dev_count), ctx->sm_count, s);

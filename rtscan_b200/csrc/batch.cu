@@ -1419,7 +1419,7 @@ bool always_true(uint2 term) { return term.x == 0 && term.y == 0xFFFFFFFFu; }
 // On a 2^23-row segment of 4 columns a fused scan takes about 5.6 us plus
 // 5.9 us per term; two queries of 1, 2 and 3 columns each took 17, 28 and
 // 41 us as fused scans (4 columns each: 55 us), a few-query pass of two to
-// eight queries over 4 columns 42-45 us.
+// eight queries over 4 columns 33-45 us.
 bool fused_each(const FewPass &f) {
   if (f.nq > 3) return false;
   int terms = 0;

@@ -242,6 +242,7 @@ struct rts_ctx {
   // scratch for the separate-pass path and the BinDex planner
   std::vector<uint32_t *> scratch_bm;
   uint64_t scratch_words = 0;
+  cudaEvent_t scratch_done = nullptr;  // after the last separate-pass scan's use of scratch_bm[0]
   void *plan_dev = nullptr;
   size_t plan_bytes = 0;
   void *plan_host = nullptr;  // pinned
