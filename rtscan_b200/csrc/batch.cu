@@ -994,12 +994,14 @@ int pass_groups(int nq) { return nq <= 128 ? 4 : nq <= 256 ? 8 : 16; }
 // Bucket shape of a column's sorted distinct boundaries B (pc.m, origin, M,
 // L, nbk) with at most max_buckets buckets, the last one past every
 // boundary (values above them all need no search).  Candidates: linear
-// buckets, and log-linear ones of M = 2, 5, 8 and 11 with the smallest L that
-// fits, then the best M's neighbours; the one with the fewest search steps
-// per row wins, fewer buckets on a tie.  Query bounds sit at value quantiles, so every interval between
-// neighbouring boundaries stands for the same share of the rows, spread
-// evenly over its values: a bucket with boundaries inside costs their search
-// steps times the shares of the intervals that it overlaps.
+// buckets, and log-linear ones of M = 2, 5 and 8 with the smallest L that
+// fits, then the values of M beside the best one for as long as they are
+// better (in M the cost falls until the buckets run out, then rises); the one
+// with the fewest search steps per row wins, fewer buckets on a tie.  Query
+// bounds sit at value quantiles, so every interval between neighbouring
+// boundaries stands for the same share of the rows, spread evenly over its
+// values: a bucket with boundaries inside costs their search steps times the
+// shares of the intervals that it overlaps.
 void pre_shape(const std::vector<uint32_t> &B, PreCol &pc, uint32_t max_buckets) {
   const uint32_t m = (uint32_t)B.size();
   pc.m = m;
@@ -1074,11 +1076,16 @@ void pre_shape(const std::vector<uint32_t> &B, PreCol &pc, uint32_t max_buckets)
       best_i = i;
     }
   };
-  for (const int i : {8, 0, 5, 11, 2}) consider(i);
-  const int near = best_i;
-  if (near > 0) {  // the next values of M
-    consider(near - 1);
-    if (near < 12) consider(near + 1);
+  for (const int i : {8, 0, 5, 2}) consider(i);
+  const int coarse = best_i;
+  if (coarse == 0) {  // (with more of M the buckets become the linear ones)
+    consider(9);
+  } else {  // up from the best M while it gets better, else down
+    for (int i = coarse + 1; i <= 12; i++) {
+      consider(i);
+      if (best_i != i) break;
+    }
+    for (int i = coarse - 1; i >= 1 && best_i == i + 1; i--) consider(i);
   }
   pc = best;
 }
